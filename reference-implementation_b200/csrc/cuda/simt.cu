@@ -1,6 +1,9 @@
-// Tiled CUDA-core GEMM (binary32 / binary64, real or complex): the plain GPU
-// path for large contractions that the tensor cores do not take (F32F32
-// without split mode, F64F64, DEFAULT on float/double/complex data).
+// CUDA-core products in the turned L/M/N/K view. k_simt is the tiled GEMM for
+// operands that are converted as they are loaded (storage other than the
+// compute type, complex operands rounded to 16 bits, more than 8 modes in an
+// index class or coordinates beyond 31 bits); operands stored as they are
+// computed with go to k_tile (tile.cu), and narrow products to the kernels
+// further down.
 // Complex operands keep real and imaginary planes in shared memory and
 // accumulate with four FMAs per product; op_A/op_B conjugation is applied at
 // load, op_C and op_D in the epilogue.
@@ -25,17 +28,10 @@
 #include <cstdio>
 #include <cstring>
 
-#include "tb_common.cuh"
+#include "simt.cuh"
 
 namespace tb {
 namespace simt {
-
-struct Modes {
-    int32_t n, pad;
-    int64_t ext[TB_MAXMODES];
-    int64_t s0[TB_MAXMODES];
-    int64_t s1[TB_MAXMODES];
-};
 
 __device__ __forceinline__ void decode(const Modes& m, int64_t idx, int64_t& o0, int64_t& o1)
 {
@@ -49,56 +45,11 @@ __device__ __forceinline__ void decode(const Modes& m, int64_t idx, int64_t& o0,
     }
 }
 
-struct Params {
-    const void* A;
-    const void* B;
-    const void* C;
-    void* D;
-    int32_t tA, tB, tC, tD, round_in, beta_zero, a_rows_fast, b_rows_fast;
-    int64_t M, N, K, L;
-    double alpha, beta, alpha_im, beta_im;
-    int32_t conjA, conjB, conjC, conjD, conjD_f32, d_rows_fast;
-    Modes am, ak, al;  // A: rows (M), contraction, batch (s0 = stride in A)
-    Modes bn, bk, bl;  // B: rows (N), contraction, batch (s0 = stride in B)
-    Modes cm, cn, cl;  // C (s0) and D (s1) strides of M, N, L modes
-    int32_t tiles_m, tiles_n;
-    int64_t k_chunk;   // contraction length of one split (multiple of BK)
-    void* ws;          // split sums [split][l][m][n][plane], or NULL: epilogue in place
-    int32_t a_vec, b_vec;  // operand read 16 bytes at a time (see vec_side)
-};
-
-// D = op_D(alpha * acc + beta * op_C(C)) for one element whose C value
-// (cr, ci) is already loaded (rounded, not yet conjugated)
-template <typename T, bool CPLX>
-__device__ __forceinline__ void epilogue_value(const Params& p, T xr, T xi, T cr, T ci, T& out_r, T& out_i)
-{
-    const T ar = (T)p.alpha, ai = (T)p.alpha_im, br = (T)p.beta, bi = (T)p.beta_im;
-    T vr = ar * xr - (CPLX ? ai * xi : (T)0);
-    T vi = CPLX ? ar * xi + ai * xr : (T)0;
-    if (!p.beta_zero) {
-        if (p.conjC) ci = -ci;
-        vr = fma(br, cr, vr);
-        if (CPLX) {
-            vr = fma(-bi, ci, vr);
-            vi = fma(br, ci, fma(bi, cr, vi));
-        }
-    }
-    if (p.conjD) {
-        if (p.conjD_f32) {
-            vr = (T)(float)vr;
-            vi = (T)(float)vi;
-        }
-        vi = -vi;
-    }
-    out_r = vr;
-    out_i = vi;
-}
-
 template <typename T, bool CPLX>
 __device__ __forceinline__ void epilogue_store_c(const Params& p, T xr, T xi, T cr, T ci, int64_t od)
 {
     T vr, vi;
-    epilogue_value<T, CPLX>(p, xr, xi, cr, ci, vr, vi);
+    epilogue_value<T, CPLX, Params>(p, xr, xi, cr, ci, vr, vi);
     store_elem<T>(p.D, od, p.tD, vr, vi);
 }
 
@@ -2050,6 +2001,7 @@ size_t simt_scratch_bytes(const tb_plan* P)
     tb_ptrs d = {nullptr, nullptr, nullptr, nullptr};
     simt_params(P, &d, p);
     if (narrow_width(P, p)) return 0;
+    if (tile_takes(p, P->compute)) return tile_scratch_bytes(p, P->compute);
     return with_cfg(P->compute, tile_for(P->compute, p.M, p.N), [&](auto cfg) { return decltype(cfg)::split(p).ws_bytes; });
 }
 
@@ -2433,6 +2385,7 @@ cudaError_t launch_simt(const tb_plan* P, const tb_ptrs* d, cudaStream_t s)
         default: return launch_narrow_t<double, 64>(np, s);
         }
     }
+    if (tile_takes(p, P->compute)) return launch_tile(p, P->compute, s);
     return with_cfg(P->compute, tile_for(P->compute, p.M, p.N), [&](auto cfg) { return decltype(cfg)::launch(p, s); });
 }
 
