@@ -2001,7 +2001,8 @@ size_t simt_scratch_bytes(const tb_plan* P)
     tb_ptrs d = {nullptr, nullptr, nullptr, nullptr};
     simt_params(P, &d, p);
     if (narrow_width(P, p)) return 0;
-    if (tile_takes(p, P->compute)) return tile_scratch_bytes(p, P->compute);
+    // k_simt's split sums; k_tile, which needs less or none, keeps within them,
+    // so that what a budget admits does not depend on the operands' storage
     return with_cfg(P->compute, tile_for(P->compute, p.M, p.N), [&](auto cfg) { return decltype(cfg)::split(p).ws_bytes; });
 }
 
@@ -2385,7 +2386,7 @@ cudaError_t launch_simt(const tb_plan* P, const tb_ptrs* d, cudaStream_t s)
         default: return launch_narrow_t<double, 64>(np, s);
         }
     }
-    if (tile_takes(p, P->compute)) return launch_tile(p, P->compute, s);
+    if (tile_takes(p, P->compute)) return launch_tile(p, P->compute, simt_scratch_bytes(P), s);
     return with_cfg(P->compute, tile_for(P->compute, p.M, p.N), [&](auto cfg) { return decltype(cfg)::launch(p, s); });
 }
 

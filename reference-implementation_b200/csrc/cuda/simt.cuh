@@ -61,9 +61,8 @@ __device__ __forceinline__ void epilogue_value(const P& p, T xr, T xi, T cr, T c
 
 }  // namespace simt
 
-// tile.cu: the tiled GEMM over asynchronous copies
+// tile.cu: the tiled GEMM over asynchronous copies; its split sums stay within ws_limit bytes
 bool tile_takes(const simt::Params& p, int compute);
-size_t tile_scratch_bytes(const simt::Params& p, int compute);
-cudaError_t launch_tile(const simt::Params& p, int compute, cudaStream_t s);
+cudaError_t launch_tile(const simt::Params& p, int compute, size_t ws_limit, cudaStream_t s);
 
 }  // namespace tb

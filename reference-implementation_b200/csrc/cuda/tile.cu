@@ -773,8 +773,10 @@ struct Split {
 // About two blocks per SM in all. A split keeps at least two slices of the
 // contraction (less would spend more on the meeting of the ranks than on the
 // sums); a cluster serves up to 8, beyond that the workspace pays once every
-// one of 8 ranks would walk more than 16 slices.
-static Split choose_split(int64_t tiles, int64_t K, int bk, int64_t outs, size_t elem)
+// one of 8 ranks would walk more than 16 slices. ws_limit: the scratch a
+// product is charged for by a server (simt_scratch_bytes), which the
+// workspace stays within.
+static Split choose_split(int64_t tiles, int64_t K, int bk, int64_t outs, size_t elem, size_t ws_limit)
 {
     Split r = {1, 1, K, 0};
     const int64_t slices = (K + bk - 1) / bk;
@@ -784,7 +786,7 @@ static Split choose_split(int64_t tiles, int64_t K, int bk, int64_t outs, size_t
     if (want > 8 && slices > 8 * 16) {
         int64_t S = want < slices / 4 ? want : slices / 4;
         if (S > 1024) S = 1024;
-        while (S > 1 && (double)S * (double)outs * (double)elem > 256.0 * 1024 * 1024) S /= 2;
+        while (S > 1 && (double)S * (double)outs * (double)elem > (double)ws_limit) S /= 2;
         if (S > 8) {
             const int64_t per = (slices + S - 1) / S;
             r.chunk = per * bk;
@@ -800,15 +802,8 @@ static Split choose_split(int64_t tiles, int64_t K, int bk, int64_t outs, size_t
     return r;
 }
 
-template <class W>
-static Split split_of(const simt::Params& p)
-{
-    const int64_t tiles = ((p.M + W::BM - 1) / W::BM) * ((p.N + W::BN - 1) / W::BN) * p.L;
-    return choose_split(tiles, p.K, W::BK, p.L * p.M * p.N, W::E);
-}
-
 template <class W, bool RND>
-static cudaError_t launch(const simt::Params& sp, cudaStream_t s)
+static cudaError_t launch(const simt::Params& sp, size_t ws_limit, cudaStream_t s)
 {
     Params p;
     memset(&p, 0, sizeof(p));
@@ -852,7 +847,7 @@ static cudaError_t launch(const simt::Params& sp, cudaStream_t s)
     p.tiles_n = (p.N + W::BN - 1) / W::BN;
     const int64_t blocks = (int64_t)p.tiles_m * p.tiles_n * sp.L;
     if (blocks <= 0 || blocks > 0x7fffffff) return cudaErrorInvalidConfiguration;
-    const Split split = split_of<W>(sp);
+    const Split split = choose_split(blocks, sp.K, W::BK, sp.L * sp.M * sp.N, W::E, ws_limit);
     p.k_chunk = split.chunk;
     p.cluster = split.cluster;
 
@@ -942,19 +937,14 @@ bool tile_takes(const simt::Params& p, int compute)
     return true;
 }
 
-size_t tile_scratch_bytes(const simt::Params& p, int compute)
-{
-    return tile::with_tile(p, compute, [&](auto w) { return tile::split_of<decltype(w)>(p).ws_bytes; });
-}
-
-cudaError_t launch_tile(const simt::Params& p, int compute, cudaStream_t s)
+cudaError_t launch_tile(const simt::Params& p, int compute, size_t ws_limit, cudaStream_t s)
 {
     return tile::with_tile(p, compute, [&](auto w) {
         using W = decltype(w);
         if constexpr (!W::CPLX && W::E == 4) {
-            if (p.round_in != TB_ROUND_NONE) return tile::launch<W, true>(p, s);
+            if (p.round_in != TB_ROUND_NONE) return tile::launch<W, true>(p, ws_limit, s);
         }
-        return tile::launch<W, false>(p, s);
+        return tile::launch<W, false>(p, ws_limit, s);
     });
 }
 
