@@ -13,6 +13,7 @@
 // plan's compute domain (real/complex, binary32/binary64) and honour the
 // plan's operand rounding for the 16-bit precisions.
 #include <cstdio>
+#include <type_traits>
 
 #include "tb_common.cuh"
 
@@ -62,9 +63,15 @@ __device__ __forceinline__ void unary_sum(const void* base, int64_t off, int t, 
     int64_t c[TB_MAXMODES];
     for (int j = 0; j < n; j++) c[j] = 0;
     int64_t o = off;
-    for (int64_t u = 0; u < size; u++) {
-        R xr, xi;
-        load_elem<R>(base, o, t, xr, xi);
+    auto next = [&]() {
+        for (int j = 0; j < n; j++) {
+            o += str[j];
+            if (++c[j] < ext[j]) break;
+            o -= str[j] * ext[j];
+            c[j] = 0;
+        }
+    };
+    auto add = [&](R xr, R xi) {
         if (conj) xi = -xi;
         re += xr;
         im += xi;
@@ -72,17 +79,30 @@ __device__ __forceinline__ void unary_sum(const void* base, int64_t off, int t, 
             re = round_in<R>(re, rmode);
             im = round_in<R>(im, rmode);
         }
-        for (int j = 0; j < n; j++) {
-            o += str[j];
-            if (++c[j] < ext[j]) break;
-            o -= str[j] * ext[j];
-            c[j] = 0;
+    };
+    // 4 loads in flight, added in order
+    int64_t u = 0;
+    for (; u + 4 <= size; u += 4) {
+        R xr[4], xi[4];
+#pragma unroll
+        for (int v = 0; v < 4; v++) {
+            load_elem<R>(base, o, t, xr[v], xi[v]);
+            next();
         }
+#pragma unroll
+        for (int v = 0; v < 4; v++) add(xr[v], xi[v]);
+    }
+    for (; u < size; u++) {
+        R xr, xi;
+        load_elem<R>(base, o, t, xr, xi);
+        add(xr, xi);
+        next();
     }
 }
 
+// op_D(alpha * sum + beta * op_C(C)) into D, C's value (cr, ci) already loaded
 template <typename R, bool CPLX>
-__device__ __forceinline__ void finish(const GenParams& p, R sr, R si, const void* C, int64_t oC, void* D, int64_t oD)
+__device__ __forceinline__ void finish_c(const GenParams& p, R sr, R si, R cr, R ci, void* D, int64_t oD)
 {
     // alpha * sum
     R ar = (R)p.alpha_re, ai = (R)p.alpha_im;
@@ -95,8 +115,6 @@ __device__ __forceinline__ void finish(const GenParams& p, R sr, R si, const voi
         acci = 0;
     }
     if (!p.beta_zero) {
-        R cr, ci;
-        load_rounded<R>(C, oC, p.tC, p.round_in, cr, ci);
         if (p.conjC) ci = -ci;
         R br = (R)p.beta_re, bi = (R)p.beta_im;
         if (CPLX) {
@@ -114,6 +132,14 @@ __device__ __forceinline__ void finish(const GenParams& p, R sr, R si, const voi
         acci = -acci;
     }
     store_elem<R>(D, oD, p.tD, accr, acci);
+}
+
+template <typename R, bool CPLX>
+__device__ __forceinline__ void finish(const GenParams& p, R sr, R si, const void* C, int64_t oC, void* D, int64_t oD)
+{
+    R cr = 0, ci = 0;
+    if (!p.beta_zero) load_rounded<R>(C, oC, p.tC, p.round_in, cr, ci);
+    finish_c<R, CPLX>(p, sr, si, cr, ci, D, oD);
 }
 
 // offsets in A, B, C and D of the free coordinates of output index i
@@ -209,6 +235,124 @@ __global__ void __launch_bounds__(256) k_elementwise(GenParams p, const void* A,
         element<R, CPLX>(p, A, B, C, D, i);
 }
 
+// Several outputs per thread (k_element_rows) or per warp (k_warp_rows): NR
+// outputs along a free mode that one operand (the shared one) lacks. The
+// shared operand's value is loaded once per term for all of them, the index
+// arithmetic is done once, and the other operand's NR loads of a term are in
+// flight together. Every output sums the same terms in the same order as
+// element() or warp_element(), so the bits are those of the kernels that take
+// one output at a time, of the grouped launches and of the request loop.
+// One output per thread was bound by one load of the varying operand in flight
+// for each of the shared one, one per warp by index arithmetic and shuffles:
+// the 823 MB Hadamard product of 69 terms went from 621 to 197 us (4.2 TB/s),
+// its form with the contraction contiguous from 1790 to 348 us, and the
+// mixed-class product's unary sums, loads side by side, from 40 to 23 us.
+// The mode's place in p's free modes counts the groups: a group is NR
+// neighbours, or, spread, every groups-th coordinate (so that the lanes of a
+// warp still read neighbours when the mode is the one they walk).
+struct RowGroup {
+    int64_t ext, groups, inner;  // extent of the mode, its groups, outputs of p per group step
+    int64_t v, c, d;             // from one row of a group to the next: in the varying operand, C, D
+    int32_t vary_b, spread;      // the varying operand is B
+};
+
+// outputs of group index i of p
+template <int NR>
+__device__ __forceinline__ int rows_of(const RowGroup& g, int64_t i)
+{
+    const int64_t q = i / g.inner % g.groups;
+    const int64_t n = g.spread ? (g.ext - q + g.groups - 1) / g.groups : g.ext - q * NR;
+    return n < NR ? (int)n : NR;
+}
+
+// DIRECT: both operands stored as R (pairs of R for complex), no rounding
+template <typename R, bool CPLX, bool DIRECT>
+__device__ __forceinline__ void load_term(const void* base, int64_t off, int t, int rmode, R& re, R& im)
+{
+    if constexpr (DIRECT && CPLX) {
+        const R* q = (const R*)base + 2 * off;
+        re = __ldg(q);
+        im = __ldg(q + 1);
+    } else if constexpr (DIRECT) {
+        re = __ldg((const R*)base + off);
+        im = 0;
+    } else {
+        load_rounded<R>(base, off, t, rmode, re, im);
+    }
+}
+
+template <typename R, bool CPLX, bool DIRECT, int NR>
+__global__ void __launch_bounds__(256) k_element_rows(GenParams p, RowGroup g, const void* A, const void* B,
+                                                      const void* C, void* D)
+{
+    // terms whose loads are issued together: about 16 loads of the varying operand
+    constexpr int UNR = NR >= 8 ? 2 : 4;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    const void* V = g.vary_b ? B : A;
+    const void* S = g.vary_b ? A : B;
+    const int tV = g.vary_b ? p.tB : p.tA, tS = g.vary_b ? p.tA : p.tB;
+    const int conjV = g.vary_b ? p.conjB : p.conjA, conjS = g.vary_b ? p.conjA : p.conjB;
+    const int64_t* kV_s = g.vary_b ? p.K_sB : p.K_sA;
+    const int64_t* kS_s = g.vary_b ? p.K_sA : p.K_sB;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < p.sizeF; i += stride) {
+        int64_t oA, oB, oC, oD;
+        free_offsets(p, i, oA, oB, oC, oD);
+        const int rows = rows_of<NR>(g, i);
+        int64_t at[NR];  // absent outputs repeat the first one's loads
+#pragma unroll
+        for (int r = 0; r < NR; r++) at[r] = r < rows ? r * g.v : 0;
+        R sr[NR], si[NR];
+#pragma unroll
+        for (int r = 0; r < NR; r++) sr[r] = si[r] = 0;
+        int64_t kc[TB_MAXMODES];
+        for (int j = 0; j < p.nK; j++) kc[j] = 0;
+        int64_t kV = g.vary_b ? oB : oA, kS = g.vary_b ? oA : oB;
+        auto next = [&]() {
+            for (int j = 0; j < p.nK; j++) {
+                kV += kV_s[j];
+                kS += kS_s[j];
+                if (++kc[j] < p.K_ext[j]) break;
+                kV -= kV_s[j] * p.K_ext[j];
+                kS -= kS_s[j] * p.K_ext[j];
+                kc[j] = 0;
+            }
+        };
+        auto terms = [&](auto count) {
+            constexpr int U = decltype(count)::value;
+            R vr[U][NR], vi[U][NR], xr[U], xi[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                load_term<R, CPLX, DIRECT>(S, kS, tS, p.round_in, xr[u], xi[u]);
+#pragma unroll
+                for (int r = 0; r < NR; r++) load_term<R, CPLX, DIRECT>(V, kV + at[r], tV, p.round_in, vr[u][r], vi[u][r]);
+                next();
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                if (conjS) xi[u] = -xi[u];
+#pragma unroll
+                for (int r = 0; r < NR; r++) {
+                    if (conjV) vi[u][r] = -vi[u][r];
+                    if (g.vary_b) cmac<R, CPLX>(sr[r], si[r], xr[u], xi[u], vr[u][r], vi[u][r]);
+                    else cmac<R, CPLX>(sr[r], si[r], vr[u][r], vi[u][r], xr[u], xi[u]);
+                }
+            }
+        };
+        int64_t k = 0;
+        for (; k + UNR <= p.sizeK; k += UNR) terms(std::integral_constant<int, UNR>());
+        for (; k < p.sizeK; k++) terms(std::integral_constant<int, 1>());
+        R cr[NR], ci[NR];
+#pragma unroll
+        for (int r = 0; r < NR; r++) {
+            cr[r] = ci[r] = 0;
+            if (!p.beta_zero && r < rows) load_rounded<R>(C, oC + r * g.c, p.tC, p.round_in, cr[r], ci[r]);
+        }
+#pragma unroll
+        for (int r = 0; r < NR; r++)
+            if (r < rows) finish_c<R, CPLX>(p, sr[r], si[r], cr[r], ci[r], D, oD + r * g.d);
+    }
+}
+
 // One warp per element of D for products whose contraction runs along an
 // operand's contiguous mode while consecutive outputs do not (batched
 // matrix-vector and Hadamard products with A stored contraction-fastest):
@@ -279,6 +423,143 @@ __global__ void __launch_bounds__(256) k_warpdot(GenParams p, const void* A, con
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
     for (int64_t i = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < p.sizeF; i += warps)
         warp_element<R, CPLX>(p, A, B, C, D, i, threadIdx.x & 31);
+}
+
+// warp_element for NR outputs at a time (RowGroup): the partial sums of the
+// rows meet in one transposed shuffle tree, in which a lane hands away half of
+// its rows at each step, so 8 rows take 9 shuffles instead of 40 and end on 8
+// different lanes; each row's sum is that of the same tree as warp_element's.
+template <typename R, bool CPLX, bool DIRECT, int NR>
+__global__ void __launch_bounds__(256) k_warp_rows(GenParams p, RowGroup g, const void* A, const void* B, const void* C,
+                                                   void* D)
+{
+    constexpr int UNR = 2;  // terms of a lane whose loads are issued together
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+    const int lane = threadIdx.x & 31;
+    const void* V = g.vary_b ? B : A;
+    const void* S = g.vary_b ? A : B;
+    const int tV = g.vary_b ? p.tB : p.tA, tS = g.vary_b ? p.tA : p.tB;
+    const int conjV = g.vary_b ? p.conjB : p.conjA, conjS = g.vary_b ? p.conjA : p.conjB;
+    const int nUV = g.vary_b ? p.nUB : p.nUA, nUS = g.vary_b ? p.nUA : p.nUB;
+    const int64_t sizeUV = g.vary_b ? p.sizeUB : p.sizeUA, sizeUS = g.vary_b ? p.sizeUA : p.sizeUB;
+    const int64_t *UV_ext = g.vary_b ? p.UB_ext : p.UA_ext, *UV_s = g.vary_b ? p.UB_s : p.UA_s;
+    const int64_t *US_ext = g.vary_b ? p.UA_ext : p.UB_ext, *US_s = g.vary_b ? p.UA_s : p.UB_s;
+    const int64_t* kV_s = g.vary_b ? p.K_sB : p.K_sA;
+    const int64_t* kS_s = g.vary_b ? p.K_sA : p.K_sB;
+    for (int64_t i = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < p.sizeF; i += warps) {
+        int64_t oA, oB, oC, oD;
+        free_offsets(p, i, oA, oB, oC, oD);
+        const int64_t oV = g.vary_b ? oB : oA, oS = g.vary_b ? oA : oB;
+        const int rows = rows_of<NR>(g, i);
+        int64_t at[NR];  // absent outputs repeat the first one's loads
+#pragma unroll
+        for (int r = 0; r < NR; r++) at[r] = r < rows ? r * g.v : 0;
+        R sr[NR], si[NR];
+#pragma unroll
+        for (int r = 0; r < NR; r++) sr[r] = si[r] = 0;
+        auto term_offsets = [&](int64_t k, int64_t& kV, int64_t& kS) {
+            kV = oV;
+            kS = oS;
+            uint32_t r = (uint32_t)k;
+            for (int j = 0; j < p.nK; j++) {
+                const uint32_t q = j + 1 < p.nK ? fdiv(r, p.fK[j]) : 0;
+                const int64_t c = j + 1 < p.nK ? (int64_t)(r - q * p.fK[j].d) : (int64_t)r;
+                r = q;
+                kV += c * kV_s[j];
+                kS += c * kS_s[j];
+            }
+        };
+        auto add = [&](int r, R vr, R vi, R xr, R xi) {
+            if (g.vary_b) cmac<R, CPLX>(sr[r], si[r], xr, xi, vr, vi);
+            else cmac<R, CPLX>(sr[r], si[r], vr, vi, xr, xi);
+        };
+        int64_t k = lane;
+        if (nUV == 0 && nUS == 0) {
+            for (; k < p.sizeK; k += UNR * 32) {
+                R vr[UNR][NR], vi[UNR][NR], xr[UNR], xi[UNR];
+#pragma unroll
+                for (int u = 0; u < UNR; u++) {
+                    if (k + 32 * u >= p.sizeK) continue;
+                    int64_t kV, kS;
+                    term_offsets(k + 32 * u, kV, kS);
+                    load_term<R, CPLX, DIRECT>(S, kS, tS, p.round_in, xr[u], xi[u]);
+#pragma unroll
+                    for (int r = 0; r < NR; r++)
+                        load_term<R, CPLX, DIRECT>(V, kV + at[r], tV, p.round_in, vr[u][r], vi[u][r]);
+                }
+#pragma unroll
+                for (int u = 0; u < UNR; u++) {
+                    if (k + 32 * u >= p.sizeK) continue;
+                    if (conjS) xi[u] = -xi[u];
+#pragma unroll
+                    for (int r = 0; r < NR; r++) add(r, vr[u][r], conjV ? -vi[u][r] : vi[u][r], xr[u], xi[u]);
+                }
+            }
+        } else {
+            for (; k < p.sizeK; k += 32) {
+                int64_t kV, kS;
+                term_offsets(k, kV, kS);
+                R xr, xi, vr[NR], vi[NR];
+                unary_sum<R, CPLX>(S, kS, tS, conjS, p.round_in, nUS, sizeUS, US_ext, US_s, xr, xi);
+                if (nUV == 0) {
+#pragma unroll
+                    for (int r = 0; r < NR; r++) {
+                        load_term<R, CPLX, DIRECT>(V, kV + at[r], tV, p.round_in, vr[r], vi[r]);
+                        if (conjV) vi[r] = -vi[r];
+                    }
+                } else {
+                    // the rows' unary sums side by side, each in unary_sum's order
+#pragma unroll
+                    for (int r = 0; r < NR; r++) vr[r] = vi[r] = 0;
+                    int64_t c[TB_MAXMODES];
+                    for (int j = 0; j < nUV; j++) c[j] = 0;
+                    for (int64_t u = 0; u < sizeUV; u++) {
+                        R yr[NR], yi[NR];
+#pragma unroll
+                        for (int r = 0; r < NR; r++) load_elem<R>(V, kV + at[r], tV, yr[r], yi[r]);
+#pragma unroll
+                        for (int r = 0; r < NR; r++) {
+                            vr[r] += yr[r];
+                            vi[r] += conjV ? -yi[r] : yi[r];
+                            if (p.round_in != TB_ROUND_NONE) {
+                                vr[r] = round_in<R>(vr[r], p.round_in);
+                                vi[r] = round_in<R>(vi[r], p.round_in);
+                            }
+                        }
+                        for (int j = 0; j < nUV; j++) {
+                            kV += UV_s[j];
+                            if (++c[j] < UV_ext[j]) break;
+                            kV -= UV_s[j] * UV_ext[j];
+                            c[j] = 0;
+                        }
+                    }
+                }
+#pragma unroll
+                for (int r = 0; r < NR; r++) add(r, vr[r], vi[r], xr, xi);
+            }
+        }
+        // step o: a lane keeps the upper or lower half of its rows by its bit o
+        int row = 0, o = 16;
+#pragma unroll
+        for (int n = NR; n > 1; n /= 2, o /= 2) {
+            const bool up = (lane & o) != 0;
+            row += up ? n / 2 : 0;
+#pragma unroll
+            for (int r = 0; r < n / 2; r++) {
+                const R give = up ? sr[r] : sr[r + n / 2], keep = up ? sr[r + n / 2] : sr[r];
+                sr[r] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+                if (CPLX) {
+                    const R gi = up ? si[r] : si[r + n / 2], ki = up ? si[r + n / 2] : si[r];
+                    si[r] = ki + __shfl_xor_sync(0xffffffffu, gi, o);
+                }
+            }
+        }
+        for (; o > 0; o /= 2) {
+            sr[0] += __shfl_xor_sync(0xffffffffu, sr[0], o);
+            if (CPLX) si[0] += __shfl_xor_sync(0xffffffffu, si[0], o);
+        }
+        if (lane % (32 / NR) == 0 && row < rows) finish<R, CPLX>(p, sr[0], si[0], C, oC + row * g.c, D, oD + row * g.d);
+    }
 }
 
 // Many independent products of the same compute domain in one launch:
@@ -464,9 +745,124 @@ static bool warpdot_ok(const GenParams& g)
     return by_A || by_B;
 }
 
-template <typename R, bool CPLX>
-static cudaError_t launch_typed(const GenParams& g, int path, const tb_ptrs* d, cudaStream_t s)
+// Puts free mode j of g into groups of nr (RowGroup): neighbours, the groups
+// walked slowest, or spread, in place.
+static void group_rows(GenParams& g, RowGroup& q, int j, int nr, bool spread)
 {
+    const int64_t e = g.F_ext[j], groups = (e + nr - 1) / nr;
+    q.ext = e;
+    q.groups = groups;
+    q.spread = spread;
+    q.vary_b = g.F_sA[j] == 0;
+    const int64_t step = spread ? groups : 1, base = spread ? 1 : nr;
+    const int64_t s[4] = {g.F_sA[j], g.F_sB[j], g.F_sC[j], g.F_sD[j]};
+    q.v = step * (q.vary_b ? s[1] : s[0]);
+    q.c = step * s[2];
+    q.d = step * s[3];
+    const int64_t others = g.sizeF / e;
+    q.inner = 1;
+    int at = j;
+    if (spread) {
+        for (int i = 0; i < j; i++) q.inner *= g.F_ext[i];
+    } else {
+        q.inner = others;
+        for (; at + 1 < g.nF; at++) {
+            g.F_ext[at] = g.F_ext[at + 1];
+            g.fF[at] = g.fF[at + 1];
+            g.F_sA[at] = g.F_sA[at + 1];
+            g.F_sB[at] = g.F_sB[at + 1];
+            g.F_sC[at] = g.F_sC[at + 1];
+            g.F_sD[at] = g.F_sD[at + 1];
+        }
+    }
+    g.F_ext[at] = groups;
+    g.fF[at] = make_fastdiv(g.small_F ? (uint32_t)groups : 1u);
+    g.F_sA[at] = s[0] * base;
+    g.F_sB[at] = s[1] * base;
+    g.F_sC[at] = s[2] * base;
+    g.F_sD[at] = s[3] * base;
+    g.sizeF = others * groups;
+}
+
+static bool one_operand_lacks(const GenParams& g, int j) { return (g.F_sA[j] == 0) != (g.F_sB[j] == 0); }
+
+// Rows per thread of k_element_rows, or 1 for k_elementwise: a mode that one
+// operand lacks, other than the walk's first one (whose neighbours the lanes
+// of a warp read), and of several the one along which D is nearest; where
+// only the first one qualifies, spread over it as long as 8 neighbours are
+// left to the lanes (32 bytes of binary32). 8 or 4 rows as long as the threads
+// fill the GPU about once (148 x 1024) and the mode half a group.
+static int thread_rows(GenParams& g, RowGroup& q)
+{
+    if (g.nUA || g.nUB || g.sizeK < 1) return 1;
+    int best = -1;
+    auto a = [](int64_t x) { return x < 0 ? -x : x; };
+    for (int j = 1; j < g.nF; j++)
+        if (one_operand_lacks(g, j) && 2 * g.F_ext[j] >= 4 && (best < 0 || a(g.F_sD[j]) < a(g.F_sD[best]))) best = j;
+    const bool spread = best < 0;
+    if (spread) {
+        if (g.nF < 1 || !one_operand_lacks(g, 0)) return 1;
+        best = 0;
+    }
+    const int64_t e = g.F_ext[best], others = g.sizeF / e;
+    for (int nr = 8; nr >= 4; nr /= 2) {
+        const int64_t groups = (e + nr - 1) / nr;
+        if (2 * e < nr || others * groups < 148 * 1024 || (spread && groups < 8)) continue;
+        group_rows(g, q, best, nr, spread);
+        return nr;
+    }
+    return 1;
+}
+
+// Rows per warp of k_warp_rows, or 1 for k_warpdot: the mode that one operand
+// lacks and that leaves the fewest loads per output (the shared operand's
+// count an eighth), of equal ones the nearest in D. 8 or 4 rows as long as 8 warps per
+// SM have work and the mode fills half a group.
+static int warp_rows(GenParams& g, RowGroup& q)
+{
+    int best = -1;
+    double best_cost = 0;
+    auto a = [](int64_t x) { return x < 0 ? -x : x; };
+    for (int j = 0; j < g.nF; j++) {
+        if (!one_operand_lacks(g, j) || 2 * g.F_ext[j] < 4) continue;
+        const double uv = (double)(g.F_sA[j] ? g.sizeUA : g.sizeUB), us = (double)(g.F_sA[j] ? g.sizeUB : g.sizeUA);
+        const double fill = g.F_ext[j] < 8 ? (double)g.F_ext[j] : 8.0;
+        const double cost = uv + us / fill;
+        if (best < 0 || cost < best_cost || (cost == best_cost && a(g.F_sD[j]) < a(g.F_sD[best]))) {
+            best = j;
+            best_cost = cost;
+        }
+    }
+    if (best < 0) return 1;
+    const int64_t e = g.F_ext[best], others = g.sizeF / e;
+    for (int nr = 8; nr >= 4; nr /= 2) {
+        if (2 * e < nr || others * ((e + nr - 1) / nr) < 148 * 8) continue;
+        group_rows(g, q, best, nr, false);
+        return nr;
+    }
+    return 1;
+}
+
+template <typename R, bool CPLX, bool DIRECT>
+static void launch_rows(const GenParams& g, const RowGroup& q, int nr, const tb_ptrs* d, cudaStream_t s)
+{
+    if (g.warp) {
+        int64_t blocks = (g.sizeF + 7) / 8;
+        if (blocks > 148 * 32) blocks = 148 * 32;
+        if (nr == 8) k_warp_rows<R, CPLX, DIRECT, 8><<<(unsigned)blocks, 256, 0, s>>>(g, q, d->A, d->B, d->C, d->D);
+        else k_warp_rows<R, CPLX, DIRECT, 4><<<(unsigned)blocks, 256, 0, s>>>(g, q, d->A, d->B, d->C, d->D);
+        return;
+    }
+    int64_t blocks = (g.sizeF + 255) / 256;
+    if (blocks > 148 * 64) blocks = 148 * 64;
+    if (nr == 8) k_element_rows<R, CPLX, DIRECT, 8><<<(unsigned)blocks, 256, 0, s>>>(g, q, d->A, d->B, d->C, d->D);
+    else k_element_rows<R, CPLX, DIRECT, 4><<<(unsigned)blocks, 256, 0, s>>>(g, q, d->A, d->B, d->C, d->D);
+}
+
+template <typename R, bool CPLX>
+static cudaError_t launch_typed(GenParams& g, int path, const tb_ptrs* d, cudaStream_t s)
+{
+    constexpr int stored = sizeof(R) == 4 ? (CPLX ? T_C32 : T_F32) : (CPLX ? T_C64 : T_F64);
     if (path == TB_PATH_REDUCE && g.sizeK < (1ll << 31)) {
         const int S = reduce_chunks(g.sizeF, g.sizeK);
         int64_t bx = g.sizeF < 148 * 16 ? g.sizeF : 148 * 16;
@@ -493,6 +889,13 @@ static cudaError_t launch_typed(const GenParams& g, int path, const tb_ptrs* d, 
         count_launch(2);
         cudaFreeAsync(ws, s);
         return e;
+    }
+    RowGroup q;
+    memset(&q, 0, sizeof(q));
+    const int nr = g.warp ? warp_rows(g, q) : thread_rows(g, q);
+    if (nr > 1) {
+        if (g.tA == stored && g.tB == stored && g.round_in == TB_ROUND_NONE) launch_rows<R, CPLX, true>(g, q, nr, d, s);
+        else launch_rows<R, CPLX, false>(g, q, nr, d, s);
     } else if (g.warp) {
         int64_t blocks = (g.sizeF + 7) / 8;  // 8 warps, one output each
         if (blocks > 148 * 32) blocks = 148 * 32;
