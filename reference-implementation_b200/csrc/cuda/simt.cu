@@ -2338,13 +2338,20 @@ static cudaError_t launch_narrow_c(simt::NarrowParams& np, cudaStream_t s)
     return cudaGetLastError();
 }
 
+// the narrow kernel of a turned view of padded width nb (tbk_simt_kernel's codes)
+static int narrow_kind(const tb_plan* P, const simt::Params& p, int nb)
+{
+    if (P->compute == TB_C32) return cvec_ok(p, nb) ? 6 : 4;
+    return narrow_choice(p, nb, P->compute == TB_R32 ? 4 : 8).kind;
+}
+
 cudaError_t launch_simt(const tb_plan* P, const tb_ptrs* d, cudaStream_t s)
 {
     using namespace simt;
     Params p;
     simt_params(P, d, p);
     const int nb = narrow_width(P, p);
-    if (nb) {
+    if (nb && !tile_over_narrow(p, P->compute, narrow_kind(P, p, nb))) {
         NarrowParams np;
         memset(&np, 0, sizeof(np));
         np.p = p;
@@ -2406,6 +2413,6 @@ extern "C" int tbk_simt_kernel(const tb_plan* P)
     simt_params(P, &d, p);
     const int nb = narrow_width(P, p);
     if (!nb) return 0;
-    if (P->compute == TB_C32) return cvec_ok(p, nb) ? 6 : 4;
-    return narrow_choice(p, nb, P->compute == TB_R32 ? 4 : 8).kind;
+    const int kind = narrow_kind(P, p, nb);
+    return tb::tile_over_narrow(p, P->compute, kind) ? 0 : kind;
 }

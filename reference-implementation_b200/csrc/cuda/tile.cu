@@ -38,15 +38,15 @@
 // the same bits in every run, alone or served.
 #include <cstdio>
 #include <cstring>
+#include <type_traits>
 
 #include "simt.cuh"
 
 namespace tb {
 namespace tile {
 
-constexpr int NT = 256;        // threads of a block
 constexpr int MAXM = 8;        // modes per index class (more: k_simt)
-constexpr int BATCH = 8;       // slices per refill of the offset tables
+constexpr int BATCH = 4;       // slices per refill of the offset tables
 
 struct Map1 {  // coordinates of one index class -> offset in one operand
     int32_t n, pad;
@@ -59,7 +59,7 @@ struct Map2 {  // ... -> offsets in C and D
     int64_t c[MAXM], d[MAXM];
 };
 
-enum { COPY_VEC, COPY_ROWS, COPY_K };  // how an operand tile is copied (above)
+enum { COPY_VEC, COPY_PAIR, COPY_ROWS, COPY_K };  // how an operand tile is copied (above)
 
 struct Params {
     const void* A;
@@ -114,46 +114,60 @@ __device__ __forceinline__ void copy_async(uint32_t dst, const void* src, bool i
 }
 
 // The elements (kk, r) of a ROWS x BK operand slice that thread t copies, each
-// call of f covering VEC elements along the rows
-template <int E, int ROWS, int BK, typename F>
+// call of f covering a group along the rows
+template <int NT, int E, int ROWS, int BK, typename F>
 __device__ __forceinline__ void for_own(int mode, int t, F&& f)
 {
-    if (mode == COPY_VEC) {
-        constexpr int G = ROWS * E / 16;  // groups along the rows
+    if (mode == COPY_VEC || mode == COPY_PAIR) {
+        auto groups = [&](auto n) {
+            constexpr int N = decltype(n)::value, G = ROWS / N;  // groups of N rows
 #pragma unroll
-        for (int u = 0; u < (G * BK + NT - 1) / NT; u++) {
-            const int i = t + NT * u;
-            if (G * BK % NT == 0 || i < G * BK) f(i / G, (i % G) * (16 / E));
-        }
+            for (int u = 0; u < (G * BK + NT - 1) / NT; u++) {
+                const int i = t + NT * u;
+                if (G * BK % NT == 0 || i < G * BK) f(i / G, (i % G) * N);
+            }
+        };
+        if (mode == COPY_VEC) groups(std::integral_constant<int, 16 / E>());
+        else groups(std::integral_constant<int, 2>());
     } else if (mode == COPY_ROWS) {
 #pragma unroll
-        for (int u = 0; u < ROWS * BK / NT; u++) {
+        for (int u = 0; u < (ROWS * BK + NT - 1) / NT; u++) {
             const int i = t + NT * u;
-            f(i / ROWS, i % ROWS);
+            if (ROWS * BK % NT == 0 || i < ROWS * BK) f(i / ROWS, i % ROWS);
         }
     } else {
         // KS lanes along the contraction (32 bytes), RS rows per warp
-        constexpr int KS = 32 / E, RS = 32 / KS, KB = BK / KS;
+        constexpr int KS = 32 / E, RS = 32 / KS, KB = BK / KS, UNITS = ROWS * BK / 32;
+        static_assert(BK % KS == 0 && ROWS % RS == 0, "whole units of a warp");
         const int lane = t & 31, kl = lane % KS, rl = lane / KS;
 #pragma unroll
-        for (int u = 0; u < ROWS * BK / NT; u++) {
+        for (int u = 0; u < (UNITS + NT / 32 - 1) / (NT / 32); u++) {
             const int q = (t >> 5) + (NT / 32) * u;
-            f((q % KB) * KS + kl, (q / KB) * RS + rl);
+            if (UNITS % (NT / 32) == 0 || q < UNITS) f((q % KB) * KS + kl, (q / KB) * RS + rl);
         }
     }
 }
 
 // One slice of an operand: rows < rows_in and kk < k_in exist, the rest is zero
-template <int E, int ROWS, int LD, int BK>
+template <int NT, int E, int ROWS, int LD, int BK>
 __device__ __forceinline__ void copy_slice(uint32_t dst, const char* base, const int64_t* row, const int64_t* kof,
                                            int rows_in, int k_in, int mode, int half, int t)
 {
     if (mode == COPY_VEC) {
-        for_own<E, ROWS, BK>(COPY_VEC, t, [&](int kk, int r) {
+        for_own<NT, E, ROWS, BK>(COPY_VEC, t, [&](int kk, int r) {
             const bool in = r < rows_in && kk < k_in;
             copy_async<16>(dst + (uint32_t)(kk * LD + r) * E, in ? base + (row[r] + kof[kk]) * E : base, in);
         });
         return;
+    }
+    if constexpr (E == 4) {
+        if (mode == COPY_PAIR) {
+            for_own<NT, E, ROWS, BK>(COPY_PAIR, t, [&](int kk, int r) {
+                const bool in = r < rows_in && kk < k_in;
+                copy_async<8>(dst + (uint32_t)(kk * LD + r) * E, in ? base + (row[r] + kof[kk]) * E : base, in);
+            });
+            return;
+        }
     }
     auto one = [&](int kk, int r) {
         const bool in = r < rows_in && kk < k_in;
@@ -168,8 +182,8 @@ __device__ __forceinline__ void copy_slice(uint32_t dst, const char* base, const
         }
         copy_async<E>(at, src, in);
     };
-    if (mode == COPY_ROWS) for_own<E, ROWS, BK>(COPY_ROWS, t, one);
-    else for_own<E, ROWS, BK>(COPY_K, t, one);
+    if (mode == COPY_ROWS) for_own<NT, E, ROWS, BK>(COPY_ROWS, t, one);
+    else for_own<NT, E, ROWS, BK>(COPY_K, t, one);
 }
 
 // ---------------------------------------------------------------------------
@@ -202,7 +216,7 @@ template <int BM_, int BN_, int TM, int TN, int MINB_>
 struct Real32 {
     using T = float;
     static constexpr bool CPLX = false;
-    static constexpr int BM = BM_, BN = BN_, BK = 16, STAGES = 4, E = 4, PAD = 4, MINB = MINB_;
+    static constexpr int NT = 256, BM = BM_, BN = BN_, BK = 16, STAGES = 4, E = 4, PAD = 4, MINB = MINB_;
     static constexpr int LDA = BM + PAD, LDB = BN + PAD;
     static constexpr int RT = BM / TM, CT = BN / TN, GN = TN < 4 ? TN : 4;
     static_assert(RT * CT == NT, "one register tile per thread");
@@ -276,7 +290,7 @@ template <int BM_, int BN_>
 struct Complex32 {
     using T = float;
     static constexpr bool CPLX = true;
-    static constexpr int BM = BM_, BN = BN_, BK = 16, STAGES = 3, E = 8, PAD = 4, MINB = 2;
+    static constexpr int NT = 256, BM = BM_, BN = BN_, BK = 16, STAGES = 3, E = 8, PAD = 4, MINB = 2;
     static constexpr int LDA = BM + PAD, LDB = BN + PAD;
     static constexpr int TM = 4, TN = 4, RT = BM / TM, CT = BN / TN;
     static_assert(RT * CT == NT, "one register tile per thread");
@@ -344,6 +358,142 @@ struct Complex32 {
     }
 };
 
+// The tall tiles of products with few columns (mode-n products with a small
+// rank), where the multiply-adds and the load path matter as much as in the
+// wide tile: a warp owns one group of TN columns, its lanes 8 rows each (two
+// groups of 4), so a register tile costs 8 + TN words of shared memory for 8
+// TN multiply-adds; BN is the column count rounded up to groups of 8 or 12.
+template <int CT, int TN>
+struct Slim32 {
+    using T = float;
+    static constexpr bool CPLX = false;
+    static constexpr int NT = 32 * CT, BM = 256, BN = CT * TN, BK = 8, STAGES = 4, E = 4, PAD = 4;
+    static constexpr int MINB = NT <= 96 ? 4 : NT <= 128 || (NT == 160 && TN == 8) ? 3 : 2;
+    static constexpr int LDA = BM + PAD, LDB = BN + PAD;
+    uint64_t acc[4][TN / 2][2];
+    int row, col;
+
+    __device__ __forceinline__ void start(int t)
+    {
+        row = (t & 31) * 4;
+        col = (t >> 5) * TN;
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int j = 0; j < TN / 2; j++) acc[i][j][0] = acc[i][j][1] = 0;
+    }
+    __device__ __forceinline__ void slice(const char* As, const char* Bs, int kn, int)
+    {
+        const float* a_at = (const float*)As + row;
+        const float* b_at = (const float*)Bs + col;
+#pragma unroll 4
+        for (int kk = 0; kk < kn; kk++) {
+            uint64_t a[4], as[4], b[TN / 2];
+            const ulonglong2 q0 = *(const ulonglong2*)(a_at + kk * LDA), q1 = *(const ulonglong2*)(a_at + kk * LDA + 128);
+            a[0] = q0.x;
+            a[1] = q0.y;
+            a[2] = q1.x;
+            a[3] = q1.y;
+#pragma unroll
+            for (int j = 0; j < TN; j += 4) {
+                const ulonglong2 q = *(const ulonglong2*)(b_at + kk * LDB + j);
+                b[j / 2] = q.x;
+                b[j / 2 + 1] = q.y;
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++) as[i] = swapped(a[i]);
+#pragma unroll
+            for (int j = 0; j < TN / 2; j++)
+#pragma unroll
+                for (int h = 0; h < 2; h++)
+#pragma unroll
+                    for (int u = 0; u < 4; u++) {
+                        const int i = h ? 3 - u : u;
+                        fma_pair(acc[i][j][h], h ? as[i] : a[i], b[j]);
+                    }
+        }
+    }
+    template <typename F>
+    __device__ __forceinline__ void each(int, F&& put)
+    {
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int j = 0; j < TN / 2; j++) {
+                const int r = row + (i / 2) * 128 + (i % 2) * 2, c = col + 2 * j;
+                put(r, c, lo_of(acc[i][j][0]));
+                put(r + 1, c + 1, hi_of(acc[i][j][0]));
+                put(r + 1, c, lo_of(acc[i][j][1]));
+                put(r, c + 1, hi_of(acc[i][j][1]));
+            }
+    }
+};
+
+// ... of complex binary32: 4 rows (two groups of 2) and 8 columns a thread
+template <int CT>
+struct SlimComplex32 {
+    using T = float;
+    static constexpr bool CPLX = true;
+    static constexpr int NT = 32 * CT, BM = 128, BN = CT * 8, BK = 8, STAGES = 4, E = 8, PAD = 4;
+    static constexpr int MINB = NT <= 96 ? 4 : NT <= 128 ? 3 : 2;
+    static constexpr int LDA = BM + PAD, LDB = BN + PAD;
+    uint64_t acc[4][8];
+    int row, col;
+
+    __device__ __forceinline__ void start(int t)
+    {
+        row = (t & 31) * 2;
+        col = (t >> 5) * 8;
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int j = 0; j < 8; j++) acc[i][j] = 0;
+    }
+    __device__ __forceinline__ void slice(const char* As, const char* Bs, int kn, int conjA)
+    {
+        const float2* a_at = (const float2*)As + row;
+        const float2* b_at = (const float2*)Bs + col;
+        const uint32_t s_re = conjA ? 0u : 0x80000000u, s_im = conjA ? 0x80000000u : 0u;
+#pragma unroll 2
+        for (int kk = 0; kk < kn; kk++) {
+            uint64_t ar[4], ai[4];
+#pragma unroll
+            for (int i = 0; i < 4; i += 2) {
+                const float4 q = *(const float4*)(a_at + kk * LDA + (i / 2) * 64);
+                const uint32_t x = __float_as_uint(q.x), y = __float_as_uint(q.y), z = __float_as_uint(q.z),
+                               w = __float_as_uint(q.w);
+                ar[i] = pack2(x, x);
+                ar[i + 1] = pack2(z, z);
+                ai[i] = pack2(y ^ s_re, y ^ s_im);
+                ai[i + 1] = pack2(w ^ s_re, w ^ s_im);
+            }
+#pragma unroll
+            for (int j = 0; j < 8; j += 2) {
+                const ulonglong2 q = *(const ulonglong2*)(b_at + kk * LDB + j);
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const uint64_t b = h ? q.y : q.x, bs = swapped(b);
+#pragma unroll
+                    for (int i = 0; i < 4; i++) fma_pair(acc[i][j + h], ar[i], b);
+#pragma unroll
+                    for (int i = 0; i < 4; i++) fma_pair(acc[3 - i][j + h], ai[3 - i], bs);
+                }
+            }
+        }
+    }
+    template <typename F>
+    __device__ __forceinline__ void each(int flip, F&& put)
+    {
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                const float im = hi_of(acc[i][j]);
+                put(row + (i / 2) * 64 + i % 2, col + j, make_float2(lo_of(acc[i][j]), flip ? -im : im));
+            }
+    }
+};
+
 __device__ __forceinline__ void mma_f64(double (&c)[2], double a, double b)
 {
     asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
@@ -358,7 +508,7 @@ template <int BM_, int BN_, int WGM, int WGN, int MINB_>
 struct Real64 {
     using T = double;
     static constexpr bool CPLX = false;
-    static constexpr int BM = BM_, BN = BN_, BK = 16, STAGES = 3, E = 8, PAD = 4, MINB = MINB_;
+    static constexpr int NT = 256, BM = BM_, BN = BN_, BK = 16, STAGES = 3, E = 8, PAD = 4, MINB = MINB_;
     static constexpr int LDA = BM + PAD, LDB = BN + PAD;
     static constexpr int WM = BM / WGM, WN = BN / WGN, FM = WM / 8, FN = WN / 8;
     static_assert(WGM * WGN * 32 == NT, "8 warps");
@@ -413,7 +563,7 @@ template <int BM_, int BN_, int WGM, int WGN>
 struct Complex64 {
     using T = double;
     static constexpr bool CPLX = true;
-    static constexpr int BM = BM_, BN = BN_, BK = 16, STAGES = 3, E = 16, PAD = 2, MINB = 2;
+    static constexpr int NT = 256, BM = BM_, BN = BN_, BK = 16, STAGES = 3, E = 16, PAD = 2, MINB = 2;
     static constexpr int LDA = BM + PAD, LDB = BN + PAD;
     static constexpr int WM = BM / WGM, WN = BN / WGN, FM = WM / 8, FN = WN / 8;
     static_assert(WGM * WGN * 32 == NT, "8 warps");
@@ -535,13 +685,13 @@ __device__ __forceinline__ void load_remote(uint32_t a, double2& v)
 // RND: binary32 operands rounded to the precision's 16-bit format, by the
 // thread that copied them, once their slice has landed
 template <class W, bool RND>
-__global__ void __launch_bounds__(NT, W::MINB) k_tile(const __grid_constant__ Params p)
+__global__ void __launch_bounds__(W::NT, W::MINB) k_tile(const __grid_constant__ Params p)
 {
     using T = typename W::T;
     using VT = Value<T, W::CPLX>;
     using V = typename VT::V;
     using S = Layout<W>;
-    constexpr int BM = W::BM, BN = W::BN, BK = W::BK, STAGES = W::STAGES, E = W::E, KT = S::KT;
+    constexpr int NT = W::NT, BM = W::BM, BN = W::BN, BK = W::BK, STAGES = W::STAGES, E = W::E, KT = S::KT;
     extern __shared__ __align__(16) char smem[];
     int64_t* aRow = (int64_t*)(smem + S::BODY);
     int64_t* bRow = aRow + BM;
@@ -563,20 +713,20 @@ __global__ void __launch_bounds__(NT, W::MINB) k_tile(const __grid_constant__ Pa
     const int slices = kend > kbeg ? (int)((kend - kbeg + BK - 1) / BK) : 0;
 
     auto fill_offsets = [&](int batch) {
-        static_assert(2 * KT <= NT, "one table entry per thread");
         const int64_t k0 = kbeg + (int64_t)batch * KT;
         const int at = (batch & 1) * KT;
-        if (t < KT) {
-            if (k0 + t < kend) kA[at + t] = offset1(p.ak, (uint32_t)(k0 + t));
-        } else if (t < 2 * KT) {
-            if (k0 + t - KT < kend) kB[at + t - KT] = offset1(p.bk, (uint32_t)(k0 + t - KT));
+        for (int i = t; i < 2 * KT; i += NT) {
+            const int64_t k = k0 + i % KT;
+            if (k < kend) (i < KT ? kA : kB - KT)[at + i] = offset1(i < KT ? p.ak : p.bk, (uint32_t)k);
         }
     };
     for (int i = t; i < BM + BN; i += NT) {
         if (i < BM) aRow[i] = i < rows_a ? offset1(p.al, l) + offset1(p.am, m0 + i) : 0;
         else bRow[i - BM] = i - BM < rows_b ? offset1(p.bl, l) + offset1(p.bn, n0 + i - BM) : 0;
     }
-    if (slices) fill_offsets(0);
+    static_assert(STAGES <= BATCH, "the first slices lie in the first refill");
+    fill_offsets(0);
+    fill_offsets(1);
     __syncthreads();
 
     const uint32_t ring = smem_addr(smem);
@@ -586,38 +736,40 @@ __global__ void __launch_bounds__(NT, W::MINB) k_tile(const __grid_constant__ Pa
             const int at = ((s / BATCH) & 1) * KT + (s % BATCH) * BK;
             const int64_t left = kend - kbeg - (int64_t)s * BK;
             const int k_in = left < BK ? (int)left : BK;
-            copy_slice<E, BM, W::LDA, BK>(dst, (const char*)p.A, aRow, kA + at, rows_a, k_in, p.a_copy, p.a_half, t);
-            copy_slice<E, BN, W::LDB, BK>(dst + BK * W::LDA * E, (const char*)p.B, bRow, kB + at, rows_b, k_in, p.b_copy,
+            copy_slice<NT, E, BM, W::LDA, BK>(dst, (const char*)p.A, aRow, kA + at, rows_a, k_in, p.a_copy, p.a_half, t);
+            copy_slice<NT, E, BN, W::LDB, BK>(dst + BK * W::LDA * E, (const char*)p.B, bRow, kB + at, rows_b, k_in, p.b_copy,
                                           p.b_half, t);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-#pragma unroll
-    for (int s = 0; s < STAGES - 1; s++) issue(s);
-
-    // the offsets of C and D, while the first slices are on their way
-    for (int i = t; i < BM + BN; i += NT) {
-        int64_t oc = 0, od = 0, lc = 0, ld = 0;
-        if (i < BM) {
-            if (i < rows_a) {
-                offset2(p.cl, l, lc, ld);
-                offset2(p.cm, m0 + i, oc, od);
-            }
-            cRow[i] = oc + lc;
-            dRow[i] = od + ld;
-        } else {
-            if (i - BM < rows_b) offset2(p.cn, n0 + i - BM, oc, od);
-            cCol[i - BM] = oc;
-            dCol[i - BM] = od;
-        }
-    }
     W w;
     w.start(t);
-    for (int s = 0; s < slices; s++) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
-        char* As = smem + (s % STAGES) * S::STAGE;
+    // the first STAGES - 1 steps only copy (one place in the code issues copies)
+#pragma unroll 1
+    for (int s = 1 - STAGES; s < slices; s++) {
+        const int q = s + STAGES - 1;
+        if (s == -1) {
+            // the offsets of C and D, while the first slices are on their way
+            for (int i = t; i < BM + BN; i += NT) {
+                int64_t oc = 0, od = 0, lc = 0, ld = 0;
+                if (i < BM) {
+                    if (i < rows_a) {
+                        offset2(p.cl, l, lc, ld);
+                        offset2(p.cm, m0 + i, oc, od);
+                    }
+                    cRow[i] = oc + lc;
+                    dRow[i] = od + ld;
+                } else {
+                    if (i - BM < rows_b) offset2(p.cn, n0 + i - BM, oc, od);
+                    cCol[i - BM] = oc;
+                    dCol[i - BM] = od;
+                }
+            }
+        }
+        if (s >= 0) asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+        char* As = smem + ((s + STAGES) % STAGES) * S::STAGE;
         char* Bs = As + BK * W::LDA * E;
-        if constexpr (RND) {
+        if (RND && s >= 0) {
             auto round_own = [&](char* base, int ld, int mode) {
                 return [=](int kk, int r) {
                     float* x = (float*)base + kk * ld + r;
@@ -628,19 +780,25 @@ __global__ void __launch_bounds__(NT, W::MINB) k_tile(const __grid_constant__ Pa
                         v.z = round_in<float>(v.z, p.round_in);
                         v.w = round_in<float>(v.w, p.round_in);
                         *(float4*)x = v;
+                    } else if (mode == COPY_PAIR) {
+                        float2 v = *(float2*)x;
+                        v.x = round_in<float>(v.x, p.round_in);
+                        v.y = round_in<float>(v.y, p.round_in);
+                        *(float2*)x = v;
                     } else {
                         *x = round_in<float>(*x, p.round_in);
                     }
                 };
             };
-            for_own<E, BM, BK>(p.a_copy, t, round_own(As, W::LDA, p.a_copy));
-            for_own<E, BN, BK>(p.b_copy, t, round_own(Bs, W::LDB, p.b_copy));
+            for_own<NT, E, BM, BK>(p.a_copy, t, round_own(As, W::LDA, p.a_copy));
+            for_own<NT, E, BN, BK>(p.b_copy, t, round_own(Bs, W::LDB, p.b_copy));
         }
-        __syncthreads();  // slice s has landed; slice s - 1 has been read by all
-        const int q = s + STAGES - 1;
-        if (q % BATCH == BATCH / 2 && (q / BATCH + 1) * BATCH < slices) fill_offsets(q / BATCH + 1);
+        if (s >= 0) __syncthreads();  // slice s has landed; slice s - 1 has been read by all
+        if (s >= 0 && q % BATCH == BATCH / 2 && (q / BATCH + 1) * BATCH < slices) fill_offsets(q / BATCH + 1);
         issue(q);
-        w.slice(As, Bs, BK, p.conjA);
+        if (s < 0) continue;
+        const int64_t left = kend - kbeg - (int64_t)s * BK;
+        w.slice(As, Bs, left < BK ? (int)left : BK, p.conjA);
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
@@ -653,50 +811,79 @@ __global__ void __launch_bounds__(NT, W::MINB) k_tile(const __grid_constant__ Pa
     const int ranks = p.cluster;
     if (ranks > 1) cluster_barrier();
     else __syncthreads();
-    const int share = BM * BN / ranks;
-    const int first = ranks > 1 ? (int)blockIdx.y * share : 0;
-    constexpr int U = 4;  // outputs of a thread whose C values are loaded together
-    for (int e0 = first + t; e0 < first + share; e0 += NT * U) {
-        V x[U];
-        T cr[U], ci[U];
-        int64_t od[U];
-        bool in[U];
+    const int share = BM * BN / ranks, first = ranks > 1 ? (int)blockIdx.y * share : 0;
+    // the sum of the ranks' partial results for output (r, c), in rank order
+    auto summed = [&](int r, int c) {
+        const int at = r * sr + c * sc;
+        if (ranks == 1) return tile[at];
+        const uint32_t a = ring + (uint32_t)(at * (int)sizeof(V));
+        V x, y;
+        load_remote(remote(a, 0), x);
+        for (int z = 1; z < ranks; z++) {
+            load_remote(remote(a, z), y);
+            x = VT::sum(x, y);
+        }
+        return x;
+    };
+    auto place = [&](int e, int& r, int& c) {
+        r = by_rows ? e % BM : e / BN;
+        c = by_rows ? e / BM : e % BN;
+        return e < first + share && r < rows_a && c < rows_b;
+    };
+    constexpr int STORED = W::CPLX ? (sizeof(T) == 4 ? T_C32 : T_C64) : (sizeof(T) == 4 ? T_F32 : T_F64);
+    if (p.ws) {
+        for (int e = first + t; e < first + share; e += NT) {
+            int r, c;
+            if (place(e, r, c))
+                ((V*)p.ws)[(((int64_t)blockIdx.y * p.L + l) * p.M + m0 + r) * p.N + n0 + c] = summed(r, c);
+        }
+    } else if (p.tC == STORED && p.tD == STORED) {
+        // C and D as they are computed: the C values of U outputs loaded
+        // together. (Code for every storage type, unrolled, missed the
+        // instruction cache on each tile.)
+        constexpr int U = sizeof(V) == 4 ? 8 : 4;
+        constexpr int Q = W::CPLX ? 2 : 1;
+        const T *C = (const T*)p.C;
+        T* D = (T*)p.D;
+        for (int e0 = first + t; e0 < first + share; e0 += NT * U) {
+            V x[U];
+            T cr[U], ci[U];
+            int64_t od[U];
+            bool in[U];
 #pragma unroll
-        for (int u = 0; u < U; u++) {
-            const int e = e0 + NT * u;
-            const int r = by_rows ? e % BM : e / BN, c = by_rows ? e / BM : e % BN;
-            in[u] = e < first + share && r < rows_a && c < rows_b;
-            cr[u] = ci[u] = 0;
-            if (!in[u]) continue;
-            const int at = r * sr + c * sc;
-            if (ranks > 1) {
-                const uint32_t a = ring + (uint32_t)(at * (int)sizeof(V));
-                load_remote(remote(a, 0), x[u]);
-                for (int z = 1; z < ranks; z++) {
-                    V y;
-                    load_remote(remote(a, z), y);
-                    x[u] = VT::sum(x[u], y);
+            for (int u = 0; u < U; u++) {
+                int r, c;
+                in[u] = place(e0 + NT * u, r, c);
+                cr[u] = ci[u] = 0;
+                if (!in[u]) continue;
+                od[u] = Q * (dRow[r] + dCol[c]);
+                if (!p.beta_zero) {
+                    const int64_t oc = Q * (cRow[r] + cCol[c]);
+                    cr[u] = C[oc];
+                    if (W::CPLX) ci[u] = C[oc + Q - 1];
                 }
-            } else {
-                x[u] = tile[at];
+                x[u] = summed(r, c);
             }
-            if (p.ws) {
-                od[u] = (((int64_t)blockIdx.y * p.L + l) * p.M + m0 + r) * p.N + n0 + c;
-            } else {
-                od[u] = dRow[r] + dCol[c];
-                if (!p.beta_zero) load_rounded<T>(p.C, cRow[r] + cCol[c], p.tC, p.round_in, cr[u], ci[u]);
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                if (!in[u]) continue;
+                if (RND) cr[u] = round_in<T>(cr[u], p.round_in);
+                T vr, vi;
+                simt::epilogue_value<T, W::CPLX, Params>(p, VT::re(x[u]), VT::im(x[u]), cr[u], ci[u], vr, vi);
+                D[od[u]] = vr;
+                if (W::CPLX) D[od[u] + Q - 1] = vi;
             }
         }
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-            if (!in[u]) continue;
-            if (p.ws) {
-                ((V*)p.ws)[od[u]] = x[u];
-                continue;
-            }
-            T vr, vi;
-            simt::epilogue_value<T, W::CPLX, Params>(p, VT::re(x[u]), VT::im(x[u]), cr[u], ci[u], vr, vi);
-            store_elem<T>(p.D, od[u], p.tD, vr, vi);
+    } else {
+#pragma unroll 1
+        for (int e = first + t; e < first + share; e += NT) {
+            int r, c;
+            if (!place(e, r, c)) continue;
+            const V x = summed(r, c);
+            T cr = 0, ci = 0, vr, vi;
+            if (!p.beta_zero) load_rounded<T>(p.C, cRow[r] + cCol[c], p.tC, p.round_in, cr, ci);
+            simt::epilogue_value<T, W::CPLX, Params>(p, VT::re(x), VT::im(x), cr, ci, vr, vi);
+            store_elem<T>(p.D, dRow[r] + dCol[c], p.tD, vr, vi);
         }
     }
     if (ranks > 1) cluster_barrier();  // no block leaves while its tile may be read
@@ -748,12 +935,13 @@ static void map2(Map2& m, const simt::Modes& s)
     }
 }
 
-// Whether groups of w neighbouring rows are 16 aligned bytes: the first row
-// mode has stride 1 and an extent divisible by w, and every other stride and
-// the base keep the alignment.
-static bool rows_in_vectors(const simt::Modes& rows, const simt::Modes& ks, const simt::Modes& ls, const void* base, int w)
+// Whether groups of w neighbouring rows are `bytes` aligned bytes: the first
+// row mode has stride 1 and an extent divisible by w, and every other stride
+// and the base keep the alignment.
+static bool rows_in_groups(const simt::Modes& rows, const simt::Modes& ks, const simt::Modes& ls, const void* base, int w,
+                           int bytes)
 {
-    if ((uintptr_t)base % 16 || rows.n < 1 || rows.s0[0] != 1 || rows.ext[0] % w) return false;
+    if ((uintptr_t)base % (unsigned)bytes || rows.n < 1 || rows.s0[0] != 1 || rows.ext[0] % w) return false;
     for (int j = 1; j < rows.n; j++)
         if (rows.s0[j] % w) return false;
     for (int j = 0; j < ks.n; j++)
@@ -829,9 +1017,13 @@ static cudaError_t launch(const simt::Params& sp, size_t ws_limit, cudaStream_t 
     p.conjD = sp.conjD;
     p.conjD_f32 = sp.conjD_f32;
     p.d_rows_fast = sp.d_rows_fast;
-    constexpr int w = 16 / W::E;
-    p.a_copy = !sp.a_rows_fast ? COPY_K : rows_in_vectors(sp.am, sp.ak, sp.al, sp.A, w) ? COPY_VEC : COPY_ROWS;
-    p.b_copy = !sp.b_rows_fast ? COPY_K : rows_in_vectors(sp.bn, sp.bk, sp.bl, sp.B, w) ? COPY_VEC : COPY_ROWS;
+    auto copy_form = [](bool rows_fast, const simt::Modes& rows, const simt::Modes& ks, const simt::Modes& ls, const void* base) {
+        if (!rows_fast) return (int)COPY_K;
+        if (rows_in_groups(rows, ks, ls, base, 16 / W::E, 16)) return (int)COPY_VEC;
+        return (int)(W::E == 4 && rows_in_groups(rows, ks, ls, base, 2, 8) ? COPY_PAIR : COPY_ROWS);
+    };
+    p.a_copy = copy_form(sp.a_rows_fast, sp.am, sp.ak, sp.al, sp.A);
+    p.b_copy = copy_form(sp.b_rows_fast, sp.bn, sp.bk, sp.bl, sp.B);
     p.a_half = W::CPLX && (uintptr_t)sp.A % W::E != 0;
     p.b_half = W::CPLX && (uintptr_t)sp.B % W::E != 0;
     map1(p.am, sp.am);
@@ -866,7 +1058,7 @@ static cudaError_t launch(const simt::Params& sp, size_t ws_limit, cudaStream_t 
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)blocks, (unsigned)(split.splits > 1 ? split.splits : split.cluster));
-    cfg.blockDim = dim3(NT);
+    cfg.blockDim = dim3(W::NT);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute at[1];
@@ -893,24 +1085,62 @@ static cudaError_t launch(const simt::Params& sp, size_t ws_limit, cudaStream_t 
     return e;
 }
 
-// Tiles by the shorter side N: the widest that N fills. Binary64 takes 128 x
-// 64 (two blocks per SM, 32 accumulators a thread); 64 x 64 where M is small.
+// Tiles by the shorter side N. Up to 64 columns: tall tiles as wide as N
+// rounded up to 8 (binary32 also to 12) where the rows fill the GPU, narrow
+// ones of 128 rows otherwise. Wider: the widest that both sides fill; binary64
+// takes 128 x 64 (two blocks per SM, 32 accumulators a thread), 64 x 64 where
+// M is small.
 template <typename F>
 static auto with_tile(const simt::Params& p, int compute, F&& f)
 {
+    const int w8 = (int)((p.N + 7) / 8);
     switch (compute) {
     case TB_R64:
-        if (p.N <= 16) return f(Real64<128, 16, 8, 1, 2>());
-        if (p.N <= 32) return f(Real64<128, 32, 4, 2, 2>());
-        if (p.M <= 64) return f(Real64<64, 64, 2, 4, 2>());
-        return f(Real64<128, 64, 4, 2, 2>());
+        if (p.N > 64) {
+            if (p.M <= 64) return f(Real64<64, 64, 2, 4, 2>());
+            return f(Real64<128, 64, 4, 2, 2>());
+        }
+        switch (w8) {
+        case 1: return f(Real64<128, 8, 8, 1, 2>());
+        case 2: return f(Real64<128, 16, 8, 1, 2>());
+        case 3: return f(Real64<128, 24, 8, 1, 2>());
+        case 4: return f(Real64<128, 32, 8, 1, 2>());
+        case 5: return f(Real64<128, 40, 8, 1, 2>());
+        case 6: return f(Real64<128, 48, 8, 1, 2>());
+        case 7: return f(Real64<128, 56, 8, 1, 2>());
+        default: return f(Real64<128, 64, 4, 2, 2>());
+        }
     case TB_C32:
+        if (p.N <= 64 && (double)p.M * (double)p.L >= 148.0 * 128) {
+            switch (w8) {
+            case 1: return f(SlimComplex32<1>());
+            case 2: return f(SlimComplex32<2>());
+            case 3: return f(SlimComplex32<3>());
+            case 4: return f(SlimComplex32<4>());
+            case 5: return f(SlimComplex32<5>());
+            case 6: return f(SlimComplex32<6>());
+            case 7: return f(SlimComplex32<7>());
+            default: return f(SlimComplex32<8>());
+            }
+        }
         if (p.N <= 32) return f(Complex32<128, 32>());
         return f(Complex32<64, 64>());
     case TB_C64:
         if (p.N <= 32) return f(Complex64<128, 32, 4, 2>());
         return f(Complex64<64, 64, 2, 4>());
     default:
+        if (p.N <= 64 && (double)p.M * (double)p.L >= 148.0 * 256) {
+            if (p.N <= 8) return f(Slim32<1, 8>());
+            if (p.N <= 12) return f(Slim32<1, 12>());
+            if (p.N <= 16) return f(Slim32<2, 8>());
+            if (p.N <= 24) return f(Slim32<2, 12>());
+            if (p.N <= 32) return f(Slim32<4, 8>());
+            if (p.N <= 36) return f(Slim32<3, 12>());
+            if (p.N <= 40) return f(Slim32<5, 8>());
+            if (p.N <= 48) return f(Slim32<4, 12>());
+            if (p.N <= 60) return f(Slim32<5, 12>());
+            return f(Slim32<8, 8>());
+        }
         if (p.N <= 16) return f(Real32<128, 16, 4, 2, 2>());
         if (p.N <= 32) return f(Real32<128, 32, 4, 4, 2>());
         if (p.M > 64 && p.N > 64 && (double)p.M * (double)p.N * (double)p.L >= 148.0 * 128 * 128)
@@ -935,6 +1165,29 @@ bool tile_takes(const simt::Params& p, int compute)
     for (int j = 0; j < 9; j++)
         if (m[j]->n > tile::MAXM) return false;
     return true;
+}
+
+// kind: the narrow kernel (simt.cu, NK_*; complex float 4 a row per thread, 6
+// row vectors). Narrow kernels walk the rows persistently with B resident and
+// win on many rows; with few of them, the serial staging of a long B and the
+// few blocks cost more than everything else, and one row per thread reads
+// eight times the shared memory per multiply-add. Measured (us, narrow / this
+// one; rows x columns x contraction):
+//   binary64 1.7M x 24 x 64 484 / 390, odd strides 554k x 37 x 201 1439 / 553,
+//     4224 x 8 x 250 45 / 8, 10^4 x 33 x 100 70 / 20
+//   row per thread, binary32 10^4 x 33 x 101 45 / 20, 1240 x 30 x 230 57 / 13,
+//     but 505k x 21 x 129 250 / 286; complex 505k x 45 x 127 901 / 829
+//   row vectors, binary32 4224 x 8 x 250 49 / 10, but 655k x 38 x 40 245 / 505;
+//     complex 4224 x 8 x 250 61 / 16
+// (contractions of up to 130 stay with the row vectors: 1 to 10 us either way).
+bool tile_over_narrow(const simt::Params& p, int compute, int kind)
+{
+    if (!tile_takes(p, compute)) return false;
+    const double rows = (double)p.M * (double)p.L;
+    if (compute == TB_R64) return p.K >= 64;
+    const bool vectors = kind >= 5;
+    if (vectors) return p.K > 130 && rows < 148.0 * 256;
+    return p.K > 64 && (compute == TB_C32 || rows < 148.0 * 1024);
 }
 
 cudaError_t launch_tile(const simt::Params& p, int compute, size_t ws_limit, cudaStream_t s)

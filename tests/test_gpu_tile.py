@@ -86,3 +86,23 @@ def test_same_bits_every_run(tapp, gpu, storage, M, N, K):
     tapp.lib.TAPP_destroy_executor(ex)
     assert got[0] == got[1] == got[2]
     assert tapp_b200.load().launches() > 0
+
+
+# the tall tiles: every width of 8 or 12 columns a group, with remainders in columns, rows and contraction, rows in
+# 16-byte groups, in pairs, alone and across the contraction
+@pytest.mark.parametrize("storage,prec", [(0, 0), (0, 6), (1, -1), (2, -1)])
+@pytest.mark.parametrize("N", [1, 8, 11, 16, 23, 31, 36, 39, 48, 59, 64])
+@pytest.mark.parametrize("M,a_t", [(38004, 0), (38002, 0), (37999, 0), (37999, 1)])
+def test_tall_products(tapp, oracle, gpu, storage, prec, N, M, a_t):
+    rng = np.random.default_rng(N + M + a_t + 10 * storage + prec)
+    A = ([131, M], [2, 0]) if a_t else ([M, 131], [0, 2])
+    case = spec_case(rng, storage, prec, (A[0], [N, 131], [M, N], [M, N]), (A[1], [1, 2], [0, 1], [0, 1]))
+    ex = simt_executor(tapp)
+    samples = np.random.default_rng(7).integers(0, M * N, 4096)
+    from helpers import run_on_device
+    run = case.copy()
+    assert run_on_device(tapp, run, ex) == 0
+    tapp.lib.TAPP_destroy_executor(ex)
+    err, D64, scale, offs = oracle.execute_f64(case.copy(), samples=samples)
+    assert err == 0
+    assert (np.abs(run.D.buf[run.D.base + offs].astype(np.complex128) - D64) <= error_bound(case, scale, D64)).all()
