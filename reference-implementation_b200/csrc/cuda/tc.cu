@@ -647,17 +647,17 @@ __global__ void __launch_bounds__(LOAD == 1 ? 512 : NTHREADS, 1)
     // integer round trip would turn every access below into a generic one)
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     uint8_t* tiles = smem;
-    uint8_t* bars = smem + STAGES * STAGE_BYTES;  // 256 bytes of barriers and flags
+    uint8_t* bars = smem + STAGES * STAGE_BYTES;  // barriers and flags
     uint64_t* full = (uint64_t*)bars;             // up to 6
     uint64_t* empty = (uint64_t*)(bars + 48);     // up to 6
     uint64_t* tfull = (uint64_t*)(bars + 96);
     uint64_t* tempty = (uint64_t*)(bars + 112);
-    uint64_t* cbar = (uint64_t*)(bars + 128);     // one per epilogue warp
+    uint64_t* cbar = (uint64_t*)(bars + 208);     // two per epilogue warp
     uint32_t* tmem_slot = (uint32_t*)(bars + 192);
     volatile int* abort_flag = (volatile int*)(bars + 196);
     volatile int* epi_ok = (volatile int*)(bars + 200);
     volatile int* epi_first = (volatile int*)(bars + 204);
-    uint8_t* staging = smem + STAGES * STAGE_BYTES + 256;
+    uint8_t* staging = smem + STAGES * STAGE_BYTES + BARS_BYTES;
     int64_t* colC = (int64_t*)staging;
     int64_t* colD = colC + BN;
 
@@ -675,7 +675,7 @@ __global__ void __launch_bounds__(LOAD == 1 ? 512 : NTHREADS, 1)
             // epilogue warp of either CTA, on the leader's barrier
             mbar_init(&tempty[a], CTA2 ? 2 * EW : ET);
         }
-        for (int w = 0; w < EW; w++) mbar_init(&cbar[w], 1);
+        for (int w = 0; w < 2 * EW; w++) mbar_init(&cbar[w], 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -1007,22 +1007,47 @@ __global__ void __launch_bounds__(LOAD == 1 ? 512 : NTHREADS, 1)
                 add_part = true;
             }
             if (EPI == EPI_TMA) {
-                // Per chunk: TMA-load the 32x32 box of C into this warp's
-                // staging box, combine with the accumulators, write D into the
-                // same box and TMA-store it. The first box of C is requested
-                // before the accumulators are ready.
+                // Boxes of 32 rows x 16 columns, two in turn per warp: TMA loads
+                // C into one while the other is combined with the
+                // accumulators and TMA-stored. Lane b handles box b's copies,
+                // so that the lanes resolve a tile's coordinates side by side.
+                // The tile's C is first brought to L2, while its MMAs still
+                // run: with one box per warp, resolved, loaded and stored one
+                // after the other, the epilogue of a short contraction took
+                // 20 us a tile and was the whole time of batched products.
                 const int ew = warp - 4;
                 float* box = (float*)(staging + ew * STAGE_EPI_BYTES);
-                int mc[5];  // tensor-map coordinates of this warp's rows
+                uint64_t* cb = cbar + 2 * ew;
+                constexpr int NBOX = 2 * (BN / 32 / CS);  // boxes of this warp's columns
+                int cc[5];  // tensor-map coordinates of this lane's box
                 {
-                    // the last mode keeps the whole quotient: rows past M give a
-                    // coordinate past the tensor map, where TMA clips the box
-                    int64_t r = row0 + q * 32;
+                    // a first mode's extent is a multiple of 32 and TMA dims fit 32 bits;
+                    // the last mode keeps the whole quotient: rows past M (columns past N)
+                    // give a coordinate past the tensor map, where TMA clips the box
+                    uint32_t r = (uint32_t)(row0 + q * 32);
+                    uint32_t n = (uint32_t)(tn * BN + (half + CS * (lane >> 1)) * 32 + (lane & 1) * 16);
+                    uint32_t lr = (uint32_t)lt;
+                    int k = 2;
                     for (int j = 0; j < e.mm.n; j++) {
-                        const int64_t c = j + 1 < e.mm.n ? r % e.mm.ext[j] : r;
-                        r /= e.mm.ext[j];
-                        mc[j] = (int)c;
+                        const uint32_t x = (uint32_t)e.mm.ext[j], d = j + 1 < e.mm.n ? r / x : 0;
+                        const int c = (int)(r - d * x);
+                        if (j == 0) cc[0] = c;
+                        else cc[k++] = c;
+                        r = d;
                     }
+                    for (int j = 0; j < e.nn.n; j++) {
+                        const uint32_t x = (uint32_t)e.nn.ext[j], d = j + 1 < e.nn.n ? n / x : 0;
+                        const int c = (int)(n - d * x);
+                        if (j == 0) cc[1] = c;
+                        else cc[k++] = c;
+                        n = d;
+                    }
+                    for (int j = 0; j < e.ll.n; j++) {
+                        const uint32_t x = (uint32_t)e.ll.ext[j], d = lr / x;
+                        cc[k++] = (int)(lr - d * x);
+                        lr = d;
+                    }
+                    while (k < 5) cc[k++] = 0;
                 }
                 // the tensor maps of this tile's batch (written to global memory
                 // before the launch: acquire them for the tensor-map proxy)
@@ -1036,43 +1061,27 @@ __global__ void __launch_bounds__(LOAD == 1 ? 512 : NTHREADS, 1)
                         asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(mapC) : "memory");
                     }
                 }
-                int lc[5];
-                {
-                    int64_t r = lt;
-                    for (int j = 0; j < e.ll.n; j++) {
-                        lc[j] = (int)(r % e.ll.ext[j]);
-                        r /= e.ll.ext[j];
-                    }
-                }
-                auto coords = [&](int ch, int (&cc)[5]) {
-                    int nc[5];
-                    int64_t r = (int64_t)tn * BN + ch * 32;
-                    for (int j = 0; j < e.nn.n; j++) {
-                        nc[j] = (int)(j + 1 < e.nn.n ? r % e.nn.ext[j] : r);
-                        r /= e.nn.ext[j];
-                    }
-                    int k = 0;
-                    cc[k++] = mc[0];
-                    cc[k++] = nc[0];
-                    for (int j = 1; j < e.mm.n; j++) cc[k++] = mc[j];
-                    for (int j = 1; j < e.nn.n; j++) cc[k++] = nc[j];
-                    for (int j = 0; j < e.ll.n; j++) cc[k++] = lc[j];
-                    while (k < 5) cc[k++] = 0;
-                };
-                const int nch = BN / 32 / CS;  // chunks per warp
                 const float alpha = e.alpha_re, beta = e.beta_re;
                 const int rmode = e.round_C;
                 const bool bzero = e.beta_zero != 0;
                 bool ok = true;
-                auto issue_c = [&](int t) {
-                    if (lane == 0 && !bzero) {
-                        int cc[5];
-                        coords(half + CS * t, cc);
-                        mbar_expect_tx(&cbar[ew], STAGE_EPI_BYTES);
-                        tma_load_5d(box, mapC, &cbar[ew], cc);
+                int issued = 0;  // boxes of C requested
+                auto issue_c = [&]() {
+                    if (lane == issued) {
+                        mbar_expect_tx(&cb[issued & 1], EPI_BOX_BYTES);
+                        tma_load_5d(box + (issued & 1) * (EPI_BOX_BYTES / 4), mapC, &cb[issued & 1], cc);
                     }
+                    issued++;
                 };
-                issue_c(0);
+                if (!bzero) {
+                    issue_c();
+                    issue_c();
+                    if (lane >= 2 && lane < NBOX && row0 + q * 32 < e.M &&
+                        (int64_t)tn * BN + (half + CS * (lane >> 1)) * 32 + (lane & 1) * 16 < e.N)
+                        asm volatile("cp.async.bulk.prefetch.tensor.5d.L2.global [%0, {%1, %2, %3, %4, %5}];" ::"l"(mapC),
+                                     "r"(cc[0]), "r"(cc[1]), "r"(cc[2]), "r"(cc[3]), "r"(cc[4])
+                                     : "memory");
+                }
                 if (!pre) {
                     if (et == 0) *epi_ok = mbar_wait(&tfull[acc], aph, abort_flag) ? 1 : 0;
                     epi_bar();
@@ -1082,7 +1091,7 @@ __global__ void __launch_bounds__(LOAD == 1 ? 512 : NTHREADS, 1)
                 }
                 fence_after();
 #pragma unroll 1
-                for (int t = 0; t < nch; t++) {
+                for (int t = 0; t < NBOX / 2; t++) {
                     const int ch = half + CS * t;
                     uint32_t r[32];
                     if (ok) tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN + ch * 32, r);
@@ -1091,34 +1100,41 @@ __global__ void __launch_bounds__(LOAD == 1 ? 512 : NTHREADS, 1)
                         for (int j = 0; j < 32; j++)
                             r[j] = __float_as_uint(__uint_as_float(r[j]) + __ldcg(&part[(ch * 32 + j) * BM + q * 32 + lane]));
                     }
-                    bool cok = true;
-                    if (!bzero) {
-                        cok = mbar_wait(&cbar[ew], epi_cphase & 1, abort_flag);
-                        cok = __all_sync(0xffffffffu, cok);
-                        epi_cphase++;
-                    }
-                    if (ok && cok) {
-                        float cv[32];
 #pragma unroll
-                        for (int j = 0; j < 32; j++) cv[j] = bzero ? 0.f : box[j * 32 + lane];
+                    for (int h = 0; h < 2; h++) {
+                        const int b = 2 * t + h;
+                        // the other box is free once its store has read it: request the next C into it
+                        if (b > 0) {
+                            if (lane == b - 1) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                            __syncwarp();
+                            if (!bzero && ok && issued == b + 1 && issued < NBOX) issue_c();
+                        }
+                        bool cok = true;
+                        if (b < issued) {
+                            cok = mbar_wait(&cb[h], (epi_cphase >> 1) & 1, abort_flag);
+                            cok = __all_sync(0xffffffffu, cok);
+                            epi_cphase++;
+                        }
+                        float* bx = box + h * (EPI_BOX_BYTES / 4) + lane;
+                        if (ok && cok) {
+                            float cv[16];
 #pragma unroll
-                        for (int j = 0; j < 32; j++)
-                            box[j * 32 + lane] = fmaf(alpha, __uint_as_float(r[j]), beta * round_in<float>(cv[j], rmode));
-                        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                            for (int j = 0; j < 16; j++) cv[j] = bzero ? 0.f : bx[j * 32];
+#pragma unroll
+                            for (int j = 0; j < 16; j++)
+                                bx[j * 32] = fmaf(alpha, __uint_as_float(r[16 * h + j]), beta * round_in<float>(cv[j], rmode));
+                            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                        }
+                        __syncwarp();
+                        if (lane == b && ok && cok) {
+                            tma_store_5d(mapD, box + h * (EPI_BOX_BYTES / 4), cc);
+                            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                        }
+                        if (!cok) ok = false;
                     }
-                    __syncwarp();
-                    if (lane == 0 && ok && cok) {
-                        int cc[5];
-                        coords(ch, cc);
-                        tma_store_5d(mapD, box, cc);
-                        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-                        // the box is reused by the next load: wait until the store has read it
-                        asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-                    }
-                    __syncwarp();
-                    if (!cok) ok = false;
-                    if (t + 1 < nch && ok) issue_c(t + 1);
                 }
+                if (lane == NBOX - 1) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                __syncwarp();
                 fence_before();
                 release_acc(acc);
                 epi_bar();
@@ -1267,7 +1283,7 @@ __global__ void __launch_bounds__(LOAD == 1 ? 512 : NTHREADS, 1)
         }
         // no early exit above: every epilogue thread takes every tile's barriers,
         // and after an expired wait the remaining waits give up at once
-        if (EPI == EPI_TMA && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+        if (EPI == EPI_TMA) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     } else if (CVT && warp >= 8) {
         // ---------------- converters: binary32 tiles -> bfloat16 hi / lo ----------------
         // Every wait is bounded; a converter that gives up stops converting,
@@ -1391,7 +1407,7 @@ static bool make_epi_map(CUtensorMap* tm, void* base, const tb_plan* P, int whic
         strides[k - 1] = strides[k - 2];
         k++;
     }
-    cuuint32_t box[5] = {32, 32, 1, 1, 1};
+    cuuint32_t box[5] = {32, EPI_BOX_COLS, 1, 1, 1};
     cuuint32_t es[5] = {1, 1, 1, 1, 1};
     return enc(tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 5, base, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
                CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,

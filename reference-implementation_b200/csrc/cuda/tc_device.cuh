@@ -35,10 +35,12 @@ constexpr int TMEM_COLS = 512;
 constexpr int EPI_WARPS = 8;                    // two warps per TMEM lane quarter
 constexpr int EPI_THREADS = EPI_WARPS * 32;
 constexpr int NTHREADS = 128 + EPI_THREADS;
-constexpr int STAGE_EPI_BYTES = 32 * 32 * 4;  // one 32x32 fp32 box per epilogue warp
+constexpr int EPI_BOX_COLS = 16, EPI_BOX_BYTES = 32 * EPI_BOX_COLS * 4;  // binary32 C/D box of 32 rows
+constexpr int STAGE_EPI_BYTES = 2 * EPI_BOX_BYTES;  // two per epilogue warp
+constexpr int BARS_BYTES = 384;  // mbarriers and flags of k_gemm
 // tiles | barriers | epilogue staging (the per-thread epilogue keeps its
 // column-offset tables in the staging area instead)
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/ + 8 * STAGE_EPI_BYTES;
+constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*align*/ + BARS_BYTES + 8 * STAGE_EPI_BYTES;
 static_assert(2 * BN * 8 <= 8 * STAGE_EPI_BYTES, "column tables fit in the staging area");
 static_assert(SMEM_BYTES <= 232448, "dynamic shared memory limit of sm_100");
 constexpr unsigned long long WAIT_NS = 4000000000ull;  // 4 s per wait
