@@ -1,10 +1,12 @@
 // CUDA-core product kernels for every shape, storage type and precision.
 //
-//   k_elementwise  one thread per element of D: decodes the free coordinates,
-//                  then walks the contracted coordinates and, inside, the
-//                  unary coordinates of A and of B. This is the reference's
-//                  loop nest (reference_implementation/src/product.c:338-399)
-//                  with the outer loop spread over threads.
+//   k_element_rows one thread per element of D, or for 4 or 8 of them along a
+//                  mode that one operand lacks: walks the contracted
+//                  coordinates and, inside, the unary coordinates of A and of
+//                  B. This is the reference's loop nest
+//                  (reference_implementation/src/product.c:338-399) with the
+//                  outer loop spread over threads.
+//   k_warp_rows    the same with a warp, its lanes along the contraction
 //   k_reduce       one block per element of D for few outputs with a long
 //                  contraction: the contracted range is split over the
 //                  block's threads and combined with warp shuffles.
@@ -14,6 +16,7 @@
 // plan's operand rounding for the 16-bit precisions.
 #include <cstdio>
 #include <type_traits>
+#include <utility>
 
 #include "tb_common.cuh"
 
@@ -227,14 +230,6 @@ __device__ __forceinline__ void element(const GenParams& p, const void* A, const
     finish<R, CPLX>(p, sr, si, C, oC, D, oD);
 }
 
-template <typename R, bool CPLX>
-__global__ void __launch_bounds__(256) k_elementwise(GenParams p, const void* A, const void* B, const void* C, void* D)
-{
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < p.sizeF; i += stride)
-        element<R, CPLX>(p, A, B, C, D, i);
-}
-
 // Several outputs per thread (k_element_rows) or per warp (k_warp_rows): NR
 // outputs along a free mode that one operand (the shared one) lacks. The
 // shared operand's value is loaded once per term for all of them, the index
@@ -244,16 +239,17 @@ __global__ void __launch_bounds__(256) k_elementwise(GenParams p, const void* A,
 // one output at a time, of the grouped launches and of the request loop.
 // One output per thread was bound by one load of the varying operand in flight
 // for each of the shared one, one per warp by index arithmetic and shuffles:
-// the 823 MB Hadamard product of 69 terms went from 621 to 197 us (4.2 TB/s),
-// its form with the contraction contiguous from 1790 to 348 us, and the
-// mixed-class product's unary sums, loads side by side, from 40 to 23 us.
+// the 823 MB Hadamard product of 69 terms went from 621 to 199 us (4.1 TB/s),
+// its form with the contraction contiguous from 1790 to 331 us, and the
+// mixed-class product's unary sums, loads side by side and offsets from tables,
+// from 40 to 17 us.
 // The mode's place in p's free modes counts the groups: a group is NR
 // neighbours, or, spread, every groups-th coordinate (so that the lanes of a
 // warp still read neighbours when the mode is the one they walk).
 struct RowGroup {
     int64_t ext, groups, inner;  // extent of the mode, its groups, outputs of p per group step
     int64_t v, c, d;             // from one row of a group to the next: in the varying operand, C, D
-    int32_t vary_b, spread;      // the varying operand is B
+    int32_t swapped, spread;     // the varying operand, A here, is the product's B
 };
 
 // outputs of group index i of p
@@ -263,94 +259,6 @@ __device__ __forceinline__ int rows_of(const RowGroup& g, int64_t i)
     const int64_t q = i / g.inner % g.groups;
     const int64_t n = g.spread ? (g.ext - q + g.groups - 1) / g.groups : g.ext - q * NR;
     return n < NR ? (int)n : NR;
-}
-
-// DIRECT: both operands stored as R (pairs of R for complex), no rounding
-template <typename R, bool CPLX, bool DIRECT>
-__device__ __forceinline__ void load_term(const void* base, int64_t off, int t, int rmode, R& re, R& im)
-{
-    if constexpr (DIRECT && CPLX) {
-        const R* q = (const R*)base + 2 * off;
-        re = __ldg(q);
-        im = __ldg(q + 1);
-    } else if constexpr (DIRECT) {
-        re = __ldg((const R*)base + off);
-        im = 0;
-    } else {
-        load_rounded<R>(base, off, t, rmode, re, im);
-    }
-}
-
-template <typename R, bool CPLX, bool DIRECT, int NR>
-__global__ void __launch_bounds__(256) k_element_rows(GenParams p, RowGroup g, const void* A, const void* B,
-                                                      const void* C, void* D)
-{
-    // terms whose loads are issued together: about 16 loads of the varying operand
-    constexpr int UNR = NR >= 8 ? 2 : 4;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    const void* V = g.vary_b ? B : A;
-    const void* S = g.vary_b ? A : B;
-    const int tV = g.vary_b ? p.tB : p.tA, tS = g.vary_b ? p.tA : p.tB;
-    const int conjV = g.vary_b ? p.conjB : p.conjA, conjS = g.vary_b ? p.conjA : p.conjB;
-    const int64_t* kV_s = g.vary_b ? p.K_sB : p.K_sA;
-    const int64_t* kS_s = g.vary_b ? p.K_sA : p.K_sB;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < p.sizeF; i += stride) {
-        int64_t oA, oB, oC, oD;
-        free_offsets(p, i, oA, oB, oC, oD);
-        const int rows = rows_of<NR>(g, i);
-        int64_t at[NR];  // absent outputs repeat the first one's loads
-#pragma unroll
-        for (int r = 0; r < NR; r++) at[r] = r < rows ? r * g.v : 0;
-        R sr[NR], si[NR];
-#pragma unroll
-        for (int r = 0; r < NR; r++) sr[r] = si[r] = 0;
-        int64_t kc[TB_MAXMODES];
-        for (int j = 0; j < p.nK; j++) kc[j] = 0;
-        int64_t kV = g.vary_b ? oB : oA, kS = g.vary_b ? oA : oB;
-        auto next = [&]() {
-            for (int j = 0; j < p.nK; j++) {
-                kV += kV_s[j];
-                kS += kS_s[j];
-                if (++kc[j] < p.K_ext[j]) break;
-                kV -= kV_s[j] * p.K_ext[j];
-                kS -= kS_s[j] * p.K_ext[j];
-                kc[j] = 0;
-            }
-        };
-        auto terms = [&](auto count) {
-            constexpr int U = decltype(count)::value;
-            R vr[U][NR], vi[U][NR], xr[U], xi[U];
-#pragma unroll
-            for (int u = 0; u < U; u++) {
-                load_term<R, CPLX, DIRECT>(S, kS, tS, p.round_in, xr[u], xi[u]);
-#pragma unroll
-                for (int r = 0; r < NR; r++) load_term<R, CPLX, DIRECT>(V, kV + at[r], tV, p.round_in, vr[u][r], vi[u][r]);
-                next();
-            }
-#pragma unroll
-            for (int u = 0; u < U; u++) {
-                if (conjS) xi[u] = -xi[u];
-#pragma unroll
-                for (int r = 0; r < NR; r++) {
-                    if (conjV) vi[u][r] = -vi[u][r];
-                    if (g.vary_b) cmac<R, CPLX>(sr[r], si[r], xr[u], xi[u], vr[u][r], vi[u][r]);
-                    else cmac<R, CPLX>(sr[r], si[r], vr[u][r], vi[u][r], xr[u], xi[u]);
-                }
-            }
-        };
-        int64_t k = 0;
-        for (; k + UNR <= p.sizeK; k += UNR) terms(std::integral_constant<int, UNR>());
-        for (; k < p.sizeK; k++) terms(std::integral_constant<int, 1>());
-        R cr[NR], ci[NR];
-#pragma unroll
-        for (int r = 0; r < NR; r++) {
-            cr[r] = ci[r] = 0;
-            if (!p.beta_zero && r < rows) load_rounded<R>(C, oC + r * g.c, p.tC, p.round_in, cr[r], ci[r]);
-        }
-#pragma unroll
-        for (int r = 0; r < NR; r++)
-            if (r < rows) finish_c<R, CPLX>(p, sr[r], si[r], cr[r], ci[r], D, oD + r * g.d);
-    }
 }
 
 // One warp per element of D for products whose contraction runs along an
@@ -417,123 +325,313 @@ __device__ __forceinline__ void warp_element(const GenParams& p, const void* A, 
     }
 }
 
-template <typename R, bool CPLX>
-__global__ void __launch_bounds__(256) k_warpdot(GenParams p, const void* A, const void* B, const void* C, void* D)
+// DIRECT: both operands stored as R (pairs of R, aligned to the pair, for
+// complex), no rounding
+template <typename R, bool CPLX, bool DIRECT>
+__device__ __forceinline__ void load_term(const void* base, int64_t off, int t, int rmode, R& re, R& im)
 {
-    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    for (int64_t i = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < p.sizeF; i += warps)
-        warp_element<R, CPLX>(p, A, B, C, D, i, threadIdx.x & 31);
+    if constexpr (DIRECT && CPLX && sizeof(R) == 4) {
+        const float2 q = __ldg((const float2*)base + off);
+        re = q.x;
+        im = q.y;
+    } else if constexpr (DIRECT && CPLX) {
+        const double2 q = __ldg((const double2*)base + off);
+        re = q.x;
+        im = q.y;
+    } else if constexpr (DIRECT) {
+        re = __ldg((const R*)base + off);
+        im = 0;
+    } else {
+        load_rounded<R>(base, off, t, rmode, re, im);
+    }
 }
 
-// warp_element for NR outputs at a time (RowGroup): the partial sums of the
-// rows meet in one transposed shuffle tree, in which a lane hands away half of
-// its rows at each step, so 8 rows take 9 shuffles instead of 40 and end on 8
-// different lanes; each row's sum is that of the same tree as warp_element's.
-template <typename R, bool CPLX, bool DIRECT, int NR>
-__global__ void __launch_bounds__(256) k_warp_rows(GenParams p, RowGroup g, const void* A, const void* B, const void* C,
-                                                   void* D)
+// The offsets of a product's contracted and unary coordinates in shared
+// memory: resolved by the block once, a coordinate per thread, where the loops
+// over them would spend some 50 instructions a term on strides in parameter
+// memory. Longer sums than the tables step through the coordinates, and so do
+// the kernels that spread a step over 8 or 4 rows and have no unary modes, to
+// which the tables gave nothing (35 to 39 us for a product of 10^6 outputs and
+// 20 terms).
+constexpr int TAB_K = 512, TAB_U = 128;
+
+__device__ __forceinline__ bool k_tabled(const GenParams& p) { return p.sizeK <= TAB_K; }
+__device__ __forceinline__ bool u_tabled(const GenParams& p) { return p.sizeUA <= TAB_U && p.sizeUB <= TAB_U; }
+
+__device__ __forceinline__ void fill_tables(const GenParams& p, int64_t* ka, int64_t* kb, int64_t* ua, int64_t* ub)
 {
-    constexpr int UNR = 2;  // terms of a lane whose loads are issued together
-    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    const int lane = threadIdx.x & 31;
-    const void* V = g.vary_b ? B : A;
-    const void* S = g.vary_b ? A : B;
-    const int tV = g.vary_b ? p.tB : p.tA, tS = g.vary_b ? p.tA : p.tB;
-    const int conjV = g.vary_b ? p.conjB : p.conjA, conjS = g.vary_b ? p.conjA : p.conjB;
-    const int nUV = g.vary_b ? p.nUB : p.nUA, nUS = g.vary_b ? p.nUA : p.nUB;
-    const int64_t sizeUV = g.vary_b ? p.sizeUB : p.sizeUA, sizeUS = g.vary_b ? p.sizeUA : p.sizeUB;
-    const int64_t *UV_ext = g.vary_b ? p.UB_ext : p.UA_ext, *UV_s = g.vary_b ? p.UB_s : p.UA_s;
-    const int64_t *US_ext = g.vary_b ? p.UA_ext : p.UB_ext, *US_s = g.vary_b ? p.UA_s : p.UB_s;
-    const int64_t* kV_s = g.vary_b ? p.K_sB : p.K_sA;
-    const int64_t* kS_s = g.vary_b ? p.K_sA : p.K_sB;
-    for (int64_t i = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < p.sizeF; i += warps) {
+    const int t = threadIdx.x, n = blockDim.x;
+    if (k_tabled(p)) {
+        for (int k = t; k < (int)p.sizeK; k += n) {
+            uint32_t r = (uint32_t)k;
+            int64_t oa = 0, ob = 0;
+            for (int j = 0; j < p.nK; j++) {
+                const uint32_t q = j + 1 < p.nK ? fdiv(r, p.fK[j]) : 0;
+                const int64_t c = j + 1 < p.nK ? (int64_t)(r - q * p.fK[j].d) : (int64_t)r;
+                r = q;
+                oa += c * p.K_sA[j];
+                ob += c * p.K_sB[j];
+            }
+            ka[k] = oa;
+            kb[k] = ob;
+        }
+    }
+    if (u_tabled(p)) {
+        auto unary = [&](int64_t* tab, int size, int nU, const int64_t* ext, const int64_t* str) {
+            for (int u = t; u < size; u += n) {
+                uint32_t r = (uint32_t)u;
+                int64_t o = 0;
+                for (int j = 0; j < nU; j++) {
+                    const uint32_t e = (uint32_t)ext[j], q = r / e;
+                    o += (int64_t)(r - q * e) * str[j];
+                    r = q;
+                }
+                tab[u] = o;
+            }
+        };
+        if (p.nUA) unary(ua, (int)p.sizeUA, p.nUA, p.UA_ext, p.UA_s);
+        if (p.nUB) unary(ub, (int)p.sizeUB, p.nUB, p.UB_ext, p.UB_s);
+    }
+    __syncthreads();
+}
+
+// unary_sum for NR rows side by side (offsets at[r] apart), from a table of
+// offsets: U coordinates' loads in flight, added in order
+template <typename R, bool CPLX, bool DIRECT, int NR, int U>
+__device__ __forceinline__ void unary_rows(const void* base, int64_t off, const int64_t (&at)[NR], int t, int conj, int rmode,
+                                           const int64_t* tab, int size, R (&re)[NR], R (&im)[NR])
+{
+#pragma unroll
+    for (int r = 0; r < NR; r++) re[r] = im[r] = 0;
+    auto some = [&](auto count, int u0) {
+        constexpr int N = decltype(count)::value;
+        R yr[N][NR], yi[N][NR];
+#pragma unroll
+        for (int u = 0; u < N; u++) {
+            const int64_t o = off + tab[u0 + u];
+#pragma unroll
+            for (int r = 0; r < NR; r++) load_term<R, CPLX, DIRECT>(base, o + at[r], t, TB_ROUND_NONE, yr[u][r], yi[u][r]);
+        }
+#pragma unroll
+        for (int u = 0; u < N; u++)
+#pragma unroll
+            for (int r = 0; r < NR; r++) {
+                re[r] += yr[u][r];
+                im[r] += conj ? -yi[u][r] : yi[u][r];
+                if (!DIRECT && rmode != TB_ROUND_NONE) {  // the 16-bit precisions keep the running sum in 16 bits
+                    re[r] = round_in<R>(re[r], rmode);
+                    im[r] = round_in<R>(im[r], rmode);
+                }
+            }
+    };
+    int u = 0;
+    for (; u + U <= size; u += U) some(std::integral_constant<int, U>(), u);
+    for (; u < size; u++) some(std::integral_constant<int, 1>(), u);
+}
+
+// One term's values: B's (shared) and the NR rows' of A (varying),
+// unary sums included, at contracted offsets kS and kV
+template <typename R, bool CPLX, bool DIRECT, int NR>
+__device__ __forceinline__ void summed_term(const GenParams& p, const void* A, const void* B, int64_t kV, int64_t kS,
+                                            const int64_t (&at)[NR], const int64_t* ua, const int64_t* ub, R (&vr)[NR],
+                                            R (&vi)[NR], R& xr, R& xi)
+{
+    if (p.nUB == 0) {
+        load_term<R, CPLX, DIRECT>(B, kS, p.tB, p.round_in, xr, xi);
+        if (p.conjB) xi = -xi;
+    } else if (u_tabled(p)) {
+        const int64_t zero[1] = {0};
+        R yr[1], yi[1];
+        unary_rows<R, CPLX, DIRECT, 1, 4>(B, kS, zero, p.tB, p.conjB, p.round_in, ub, (int)p.sizeUB, yr, yi);
+        xr = yr[0];
+        xi = yi[0];
+    } else {
+        unary_sum<R, CPLX>(B, kS, p.tB, p.conjB, p.round_in, p.nUB, p.sizeUB, p.UB_ext, p.UB_s, xr, xi);
+    }
+    if (p.nUA == 0) {
+#pragma unroll
+        for (int r = 0; r < NR; r++) {
+            load_term<R, CPLX, DIRECT>(A, kV + at[r], p.tA, p.round_in, vr[r], vi[r]);
+            if (p.conjA) vi[r] = -vi[r];
+        }
+    } else if (u_tabled(p)) {
+        unary_rows<R, CPLX, DIRECT, NR, NR == 1 ? 4 : NR == 4 || !CPLX ? 2 : 1>(A, kV, at, p.tA, p.conjA, p.round_in, ua, (int)p.sizeUA, vr, vi);
+    } else {
+#pragma unroll 1
+        for (int r = 0; r < NR; r++) {
+            R yr, yi;
+            unary_sum<R, CPLX>(A, kV + at[r], p.tA, p.conjA, p.round_in, p.nUA, p.sizeUA, p.UA_ext, p.UA_s, yr, yi);
+#pragma unroll
+            for (int q = 0; q < NR; q++)
+                if (q == r) {
+                    vr[q] = yr;
+                    vi[q] = yi;
+                }
+        }
+    }
+}
+
+// NR outputs per thread: element() for each of them (NR = 1: the plain element kernel)
+template <typename R, bool CPLX, bool DIRECT, int NR>
+__global__ void __launch_bounds__(256) k_element_rows(GenParams p, RowGroup g,
+                                                      const void* A, const void* B, const void* C, void* D)
+{
+    constexpr bool TABLES = NR == 1;
+    __shared__ int64_t ka[TABLES ? TAB_K : 1], kb[TABLES ? TAB_K : 1], ua[TABLES ? TAB_U : 1], ub[TABLES ? TAB_U : 1];
+    // terms whose loads are issued together: 8 to 16 loads of the varying operand
+    constexpr int UNR = NR >= 8 ? 2 : NR > 1 ? 4 : (CPLX || sizeof(R) == 8) ? 4 : 8;
+    if constexpr (TABLES) fill_tables(p, ka, kb, ua, ub);
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < p.sizeF; i += stride) {
         int64_t oA, oB, oC, oD;
         free_offsets(p, i, oA, oB, oC, oD);
-        const int64_t oV = g.vary_b ? oB : oA, oS = g.vary_b ? oA : oB;
-        const int rows = rows_of<NR>(g, i);
+        const int rows = NR == 1 ? 1 : rows_of<NR>(g, i);
         int64_t at[NR];  // absent outputs repeat the first one's loads
 #pragma unroll
         for (int r = 0; r < NR; r++) at[r] = r < rows ? r * g.v : 0;
         R sr[NR], si[NR];
 #pragma unroll
         for (int r = 0; r < NR; r++) sr[r] = si[r] = 0;
-        auto term_offsets = [&](int64_t k, int64_t& kV, int64_t& kS) {
-            kV = oV;
-            kS = oS;
+        int64_t kc[TB_MAXMODES], kV = oA, kS = oB;  // stepped through without a table
+        if (!TABLES || !k_tabled(p))
+            for (int j = 0; j < p.nK; j++) kc[j] = 0;
+        auto offsets = [&](int64_t k, int64_t& v, int64_t& s) {
+            if (TABLES && k_tabled(p)) {
+                v = oA + ka[k];
+                s = oB + kb[k];
+                return;
+            }
+            v = kV;
+            s = kS;
+            for (int j = 0; j < p.nK; j++) {
+                kV += p.K_sA[j];
+                kS += p.K_sB[j];
+                if (++kc[j] < p.K_ext[j]) break;
+                kV -= p.K_sA[j] * p.K_ext[j];
+                kS -= p.K_sB[j] * p.K_ext[j];
+                kc[j] = 0;
+            }
+        };
+        auto add = [&](int r, R vr, R vi, R xr, R xi) {
+            if (g.swapped) cmac<R, CPLX>(sr[r], si[r], xr, xi, vr, vi);
+            else cmac<R, CPLX>(sr[r], si[r], vr, vi, xr, xi);
+        };
+        auto terms = [&](auto count, int64_t k) {
+            constexpr int U = decltype(count)::value;
+            R vr[U][NR], vi[U][NR], xr[U], xi[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                int64_t v, s;
+                offsets(k + u, v, s);
+                load_term<R, CPLX, DIRECT>(B, s, p.tB, p.round_in, xr[u], xi[u]);
+#pragma unroll
+                for (int r = 0; r < NR; r++) load_term<R, CPLX, DIRECT>(A, v + at[r], p.tA, p.round_in, vr[u][r], vi[u][r]);
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                if (p.conjB) xi[u] = -xi[u];
+#pragma unroll
+                for (int r = 0; r < NR; r++) add(r, vr[u][r], p.conjA ? -vi[u][r] : vi[u][r], xr[u], xi[u]);
+            }
+        };
+        int64_t k = 0;
+        if (NR > 1 || (p.nUA == 0 && p.nUB == 0)) {  // (unary modes run one row a thread)
+            for (; k + UNR <= p.sizeK; k += UNR) terms(std::integral_constant<int, UNR>(), k);
+            for (; k < p.sizeK; k++) terms(std::integral_constant<int, 1>(), k);
+        } else {
+            for (; k < p.sizeK; k++) {
+                int64_t v, s;
+                offsets(k, v, s);
+                R vr[NR], vi[NR], xr, xi;
+                summed_term<R, CPLX, DIRECT, NR>(p, A, B, v, s, at, ua, ub, vr, vi, xr, xi);
+#pragma unroll
+                for (int r = 0; r < NR; r++) add(r, vr[r], vi[r], xr, xi);
+            }
+        }
+        R cr[NR], ci[NR];
+#pragma unroll
+        for (int r = 0; r < NR; r++) {
+            cr[r] = ci[r] = 0;
+            if (!p.beta_zero && r < rows) load_rounded<R>(C, oC + r * g.c, p.tC, p.round_in, cr[r], ci[r]);
+        }
+#pragma unroll
+        for (int r = 0; r < NR; r++)
+            if (r < rows) finish_c<R, CPLX>(p, sr[r], si[r], cr[r], ci[r], D, oD + r * g.d);
+    }
+}
+
+// NR outputs per warp: warp_element for each of them (NR = 1: the plain warp
+// kernel). The partial sums of the rows meet in one transposed shuffle tree,
+// in which a lane hands away half of its rows at each step, so 8 rows take 9
+// shuffles instead of 40 and end on 8 different lanes; each row's sum is that
+// of the same tree as warp_element's. UNARY: some operand has unary modes.
+template <typename R, bool CPLX, bool DIRECT, int NR, bool UNARY>
+__global__ void __launch_bounds__(128, CPLX && NR == 8 ? (sizeof(R) == 4 ? 4 : 2) : sizeof(R) == 8 ? 4 : CPLX || UNARY ? 5 : 8)
+    k_warp_rows(GenParams p, RowGroup g, const void* A, const void* B,
+                const void* C, void* D)
+{
+    __shared__ int64_t ka[UNARY ? TAB_K : 1], kb[UNARY ? TAB_K : 1], ua[UNARY ? TAB_U : 1], ub[UNARY ? TAB_U : 1];
+    constexpr int UNR = NR == 1 ? 4 : 2;  // terms of a lane whose loads are issued together
+    if constexpr (UNARY) fill_tables(p, ka, kb, ua, ub);
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+    const int lane = threadIdx.x & 31;
+    for (int64_t i = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < p.sizeF; i += warps) {
+        int64_t oA, oB, oC, oD;
+        free_offsets(p, i, oA, oB, oC, oD);
+        const int rows = NR == 1 ? 1 : rows_of<NR>(g, i);
+        int64_t at[NR];  // absent outputs repeat the first one's loads
+#pragma unroll
+        for (int r = 0; r < NR; r++) at[r] = r < rows ? r * g.v : 0;
+        R sr[NR], si[NR];
+#pragma unroll
+        for (int r = 0; r < NR; r++) sr[r] = si[r] = 0;
+        auto offsets = [&](int64_t k, int64_t& v, int64_t& s) {
+            v = oA;
+            s = oB;
+            if (UNARY && k_tabled(p)) {
+                v += ka[k];
+                s += kb[k];
+                return;
+            }
             uint32_t r = (uint32_t)k;
             for (int j = 0; j < p.nK; j++) {
                 const uint32_t q = j + 1 < p.nK ? fdiv(r, p.fK[j]) : 0;
                 const int64_t c = j + 1 < p.nK ? (int64_t)(r - q * p.fK[j].d) : (int64_t)r;
                 r = q;
-                kV += c * kV_s[j];
-                kS += c * kS_s[j];
+                v += c * p.K_sA[j];
+                s += c * p.K_sB[j];
             }
         };
         auto add = [&](int r, R vr, R vi, R xr, R xi) {
-            if (g.vary_b) cmac<R, CPLX>(sr[r], si[r], xr, xi, vr, vi);
+            if (g.swapped) cmac<R, CPLX>(sr[r], si[r], xr, xi, vr, vi);
             else cmac<R, CPLX>(sr[r], si[r], vr, vi, xr, xi);
         };
-        int64_t k = lane;
-        if (nUV == 0 && nUS == 0) {
-            for (; k < p.sizeK; k += UNR * 32) {
+        if constexpr (!UNARY) {
+            for (int64_t k = lane; k < p.sizeK; k += UNR * 32) {
                 R vr[UNR][NR], vi[UNR][NR], xr[UNR], xi[UNR];
 #pragma unroll
                 for (int u = 0; u < UNR; u++) {
                     if (k + 32 * u >= p.sizeK) continue;
-                    int64_t kV, kS;
-                    term_offsets(k + 32 * u, kV, kS);
-                    load_term<R, CPLX, DIRECT>(S, kS, tS, p.round_in, xr[u], xi[u]);
+                    int64_t v, s;
+                    offsets(k + 32 * u, v, s);
+                    load_term<R, CPLX, DIRECT>(B, s, p.tB, p.round_in, xr[u], xi[u]);
 #pragma unroll
-                    for (int r = 0; r < NR; r++)
-                        load_term<R, CPLX, DIRECT>(V, kV + at[r], tV, p.round_in, vr[u][r], vi[u][r]);
+                    for (int r = 0; r < NR; r++) load_term<R, CPLX, DIRECT>(A, v + at[r], p.tA, p.round_in, vr[u][r], vi[u][r]);
                 }
 #pragma unroll
                 for (int u = 0; u < UNR; u++) {
                     if (k + 32 * u >= p.sizeK) continue;
-                    if (conjS) xi[u] = -xi[u];
+                    if (p.conjB) xi[u] = -xi[u];
 #pragma unroll
-                    for (int r = 0; r < NR; r++) add(r, vr[u][r], conjV ? -vi[u][r] : vi[u][r], xr[u], xi[u]);
+                    for (int r = 0; r < NR; r++) add(r, vr[u][r], p.conjA ? -vi[u][r] : vi[u][r], xr[u], xi[u]);
                 }
             }
         } else {
-            for (; k < p.sizeK; k += 32) {
-                int64_t kV, kS;
-                term_offsets(k, kV, kS);
-                R xr, xi, vr[NR], vi[NR];
-                unary_sum<R, CPLX>(S, kS, tS, conjS, p.round_in, nUS, sizeUS, US_ext, US_s, xr, xi);
-                if (nUV == 0) {
-#pragma unroll
-                    for (int r = 0; r < NR; r++) {
-                        load_term<R, CPLX, DIRECT>(V, kV + at[r], tV, p.round_in, vr[r], vi[r]);
-                        if (conjV) vi[r] = -vi[r];
-                    }
-                } else {
-                    // the rows' unary sums side by side, each in unary_sum's order
-#pragma unroll
-                    for (int r = 0; r < NR; r++) vr[r] = vi[r] = 0;
-                    int64_t c[TB_MAXMODES];
-                    for (int j = 0; j < nUV; j++) c[j] = 0;
-                    for (int64_t u = 0; u < sizeUV; u++) {
-                        R yr[NR], yi[NR];
-#pragma unroll
-                        for (int r = 0; r < NR; r++) load_elem<R>(V, kV + at[r], tV, yr[r], yi[r]);
-#pragma unroll
-                        for (int r = 0; r < NR; r++) {
-                            vr[r] += yr[r];
-                            vi[r] += conjV ? -yi[r] : yi[r];
-                            if (p.round_in != TB_ROUND_NONE) {
-                                vr[r] = round_in<R>(vr[r], p.round_in);
-                                vi[r] = round_in<R>(vi[r], p.round_in);
-                            }
-                        }
-                        for (int j = 0; j < nUV; j++) {
-                            kV += UV_s[j];
-                            if (++c[j] < UV_ext[j]) break;
-                            kV -= UV_s[j] * UV_ext[j];
-                            c[j] = 0;
-                        }
-                    }
-                }
+            for (int64_t k = lane; k < p.sizeK; k += 32) {
+                int64_t v, s;
+                offsets(k, v, s);
+                R vr[NR], vi[NR], xr, xi;
+                summed_term<R, CPLX, DIRECT, NR>(p, A, B, v, s, at, ua, ub, vr, vi, xr, xi);
 #pragma unroll
                 for (int r = 0; r < NR; r++) add(r, vr[r], vi[r], xr, xi);
             }
@@ -724,7 +822,7 @@ static void fill_params(const tb_plan* P, GenParams& g)
     g.warp = warpdot_ok(g) ? 1 : 0;
 }
 
-// Element path kernel: the warp per output (k_warpdot)
+// Element path kernel: the warp per output (k_warp_rows)
 //   - when an operand is contiguous along the contraction while consecutive
 //     outputs step it by a stride other than 0 or 1 (one thread per output
 //     would read it a row apart from lane to lane), for contractions of at
@@ -745,6 +843,21 @@ static bool warpdot_ok(const GenParams& g)
     return by_A || by_B;
 }
 
+static void swap_operands(GenParams& g)
+{
+    auto swap_all = [](int64_t* a, int64_t* b) {
+        for (int j = 0; j < TB_MAXMODES; j++) std::swap(a[j], b[j]);
+    };
+    std::swap(g.tA, g.tB);
+    std::swap(g.conjA, g.conjB);
+    std::swap(g.nUA, g.nUB);
+    std::swap(g.sizeUA, g.sizeUB);
+    swap_all(g.F_sA, g.F_sB);
+    swap_all(g.K_sA, g.K_sB);
+    swap_all(g.UA_ext, g.UB_ext);
+    swap_all(g.UA_s, g.UB_s);
+}
+
 // Puts free mode j of g into groups of nr (RowGroup): neighbours, the groups
 // walked slowest, or spread, in place.
 static void group_rows(GenParams& g, RowGroup& q, int j, int nr, bool spread)
@@ -753,10 +866,13 @@ static void group_rows(GenParams& g, RowGroup& q, int j, int nr, bool spread)
     q.ext = e;
     q.groups = groups;
     q.spread = spread;
-    q.vary_b = g.F_sA[j] == 0;
+    if (g.F_sA[j] == 0) {  // the varying operand takes A's place
+        q.swapped = 1;
+        swap_operands(g);
+    }
     const int64_t step = spread ? groups : 1, base = spread ? 1 : nr;
     const int64_t s[4] = {g.F_sA[j], g.F_sB[j], g.F_sC[j], g.F_sD[j]};
-    q.v = step * (q.vary_b ? s[1] : s[0]);
+    q.v = step * s[0];
     q.c = step * s[2];
     q.d = step * s[3];
     const int64_t others = g.sizeF / e;
@@ -786,7 +902,7 @@ static void group_rows(GenParams& g, RowGroup& q, int j, int nr, bool spread)
 
 static bool one_operand_lacks(const GenParams& g, int j) { return (g.F_sA[j] == 0) != (g.F_sB[j] == 0); }
 
-// Rows per thread of k_element_rows, or 1 for k_elementwise: a mode that one
+// Rows per thread of k_element_rows, or 1: a mode that one
 // operand lacks, other than the walk's first one (whose neighbours the lanes
 // of a warp read), and of several the one along which D is nearest; where
 // only the first one qualifies, spread over it as long as 8 neighbours are
@@ -814,29 +930,28 @@ static int thread_rows(GenParams& g, RowGroup& q)
     return 1;
 }
 
-// Rows per warp of k_warp_rows, or 1 for k_warpdot: the mode that one operand
-// lacks and that leaves the fewest loads per output (the shared operand's
-// count an eighth), of equal ones the nearest in D. 8 or 4 rows as long as 8 warps per
-// SM have work and the mode fills half a group.
+// Rows per warp of k_warp_rows, or 1: 8 or 4 rows as long as 8 warps per SM
+// have work and the mode fills half a group; of the modes that one operand
+// lacks the one with the fewest loads (a group's NR of the varying operand and
+// one of the shared, over rounds of the 16 warps per SM that run at a time),
+// of equal ones the nearest in D.
 static int warp_rows(GenParams& g, RowGroup& q)
 {
-    int best = -1;
-    double best_cost = 0;
     auto a = [](int64_t x) { return x < 0 ? -x : x; };
-    for (int j = 0; j < g.nF; j++) {
-        if (!one_operand_lacks(g, j) || 2 * g.F_ext[j] < 4) continue;
-        const double uv = (double)(g.F_sA[j] ? g.sizeUA : g.sizeUB), us = (double)(g.F_sA[j] ? g.sizeUB : g.sizeUA);
-        const double fill = g.F_ext[j] < 8 ? (double)g.F_ext[j] : 8.0;
-        const double cost = uv + us / fill;
-        if (best < 0 || cost < best_cost || (cost == best_cost && a(g.F_sD[j]) < a(g.F_sD[best]))) {
-            best = j;
-            best_cost = cost;
-        }
-    }
-    if (best < 0) return 1;
-    const int64_t e = g.F_ext[best], others = g.sizeF / e;
     for (int nr = 8; nr >= 4; nr /= 2) {
-        if (2 * e < nr || others * ((e + nr - 1) / nr) < 148 * 8) continue;
+        int best = -1;
+        double best_cost = 0;
+        for (int j = 0; j < g.nF; j++) {
+            const int64_t e = g.F_ext[j], groups = g.sizeF / e * ((e + nr - 1) / nr);
+            if (!one_operand_lacks(g, j) || 2 * e < nr || groups < 148 * 8) continue;
+            const double uv = (double)(g.F_sA[j] ? g.sizeUA : g.sizeUB), us = (double)(g.F_sA[j] ? g.sizeUB : g.sizeUA);
+            const double cost = (double)((groups + 148 * 16 - 1) / (148 * 16)) * (nr * uv + us);
+            if (best < 0 || cost < best_cost || (cost == best_cost && a(g.F_sD[j]) < a(g.F_sD[best]))) {
+                best = j;
+                best_cost = cost;
+            }
+        }
+        if (best < 0) continue;
         group_rows(g, q, best, nr, false);
         return nr;
     }
@@ -846,17 +961,21 @@ static int warp_rows(GenParams& g, RowGroup& q)
 template <typename R, bool CPLX, bool DIRECT>
 static void launch_rows(const GenParams& g, const RowGroup& q, int nr, const tb_ptrs* d, cudaStream_t s)
 {
-    if (g.warp) {
-        int64_t blocks = (g.sizeF + 7) / 8;
-        if (blocks > 148 * 32) blocks = 148 * 32;
-        if (nr == 8) k_warp_rows<R, CPLX, DIRECT, 8><<<(unsigned)blocks, 256, 0, s>>>(g, q, d->A, d->B, d->C, d->D);
-        else k_warp_rows<R, CPLX, DIRECT, 4><<<(unsigned)blocks, 256, 0, s>>>(g, q, d->A, d->B, d->C, d->D);
-        return;
-    }
-    int64_t blocks = (g.sizeF + 255) / 256;
+    const int per = g.warp ? 4 : 256, threads = g.warp ? 128 : 256;  // groups and threads of a block
+    int64_t blocks = (g.sizeF + per - 1) / per;
     if (blocks > 148 * 64) blocks = 148 * 64;
-    if (nr == 8) k_element_rows<R, CPLX, DIRECT, 8><<<(unsigned)blocks, 256, 0, s>>>(g, q, d->A, d->B, d->C, d->D);
-    else k_element_rows<R, CPLX, DIRECT, 4><<<(unsigned)blocks, 256, 0, s>>>(g, q, d->A, d->B, d->C, d->D);
+    if (blocks < 1) blocks = 1;
+    void (*kern)(GenParams, RowGroup, const void*, const void*, const void*, void*);
+    if (g.warp && (g.nUA || g.nUB))
+        kern = nr == 8 ? k_warp_rows<R, CPLX, DIRECT, 8, true>
+               : nr == 4 ? k_warp_rows<R, CPLX, DIRECT, 4, true> : k_warp_rows<R, CPLX, DIRECT, 1, true>;
+    else if (g.warp)
+        kern = nr == 8 ? k_warp_rows<R, CPLX, DIRECT, 8, false>
+               : nr == 4 ? k_warp_rows<R, CPLX, DIRECT, 4, false> : k_warp_rows<R, CPLX, DIRECT, 1, false>;
+    else
+        kern = nr == 8 ? k_element_rows<R, CPLX, DIRECT, 8>
+               : nr == 4 ? k_element_rows<R, CPLX, DIRECT, 4> : k_element_rows<R, CPLX, DIRECT, 1>;
+    kern<<<(unsigned)blocks, threads, 0, s>>>(g, q, q.swapped ? d->B : d->A, q.swapped ? d->A : d->B, d->C, d->D);
 }
 
 template <typename R, bool CPLX>
@@ -893,20 +1012,11 @@ static cudaError_t launch_typed(GenParams& g, int path, const tb_ptrs* d, cudaSt
     RowGroup q;
     memset(&q, 0, sizeof(q));
     const int nr = g.warp ? warp_rows(g, q) : thread_rows(g, q);
-    if (nr > 1) {
-        if (g.tA == stored && g.tB == stored && g.round_in == TB_ROUND_NONE) launch_rows<R, CPLX, true>(g, q, nr, d, s);
-        else launch_rows<R, CPLX, false>(g, q, nr, d, s);
-    } else if (g.warp) {
-        int64_t blocks = (g.sizeF + 7) / 8;  // 8 warps, one output each
-        if (blocks > 148 * 32) blocks = 148 * 32;
-        if (blocks < 1) blocks = 1;
-        k_warpdot<R, CPLX><<<(unsigned)blocks, 256, 0, s>>>(g, d->A, d->B, d->C, d->D);
-    } else {
-        int64_t blocks = (g.sizeF + 255) / 256;
-        if (blocks > 148 * 64) blocks = 148 * 64;
-        if (blocks < 1) blocks = 1;
-        k_elementwise<R, CPLX><<<(unsigned)blocks, 256, 0, s>>>(g, d->A, d->B, d->C, d->D);
-    }
+    const uintptr_t pair = CPLX ? 2 * sizeof(R) : 1;  // complex pairs are loaded whole
+    if (g.tA == stored && g.tB == stored && g.round_in == TB_ROUND_NONE && (uintptr_t)d->A % pair == 0 && (uintptr_t)d->B % pair == 0)
+        launch_rows<R, CPLX, true>(g, q, nr, d, s);
+    else
+        launch_rows<R, CPLX, false>(g, q, nr, d, s);
     count_launch();
     return cudaGetLastError();
 }
@@ -1280,7 +1390,7 @@ cudaError_t loop_launch(void* slots_dev, void* state, int nslots, int blocks, un
 }  // namespace tb
 
 // Kernel of the element path for a plan: 0 one thread per output, 1 one warp
-// per output (k_warpdot). No device call.
+// per output (k_warp_rows). No device call.
 extern "C" int tbk_generic_kernel(const tb_plan* P)
 {
     tb::GenParams g;
