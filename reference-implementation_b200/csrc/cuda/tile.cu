@@ -102,88 +102,93 @@ __device__ __forceinline__ void offset2(const Map2& m, uint32_t i, int64_t& oc, 
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
-// copies BYTES to shared memory, or writes zeros there (src is not read then)
+// copies BYTES to shared memory, or writes zeros there (src is not read then).
+// No memory clobber: what is copied is read only after a wait and a barrier,
+// and the offset tables may stay in registers across copies.
 template <int BYTES>
-__device__ __forceinline__ void copy_async(uint32_t dst, const void* src, bool in)
+__device__ __forceinline__ void copy_async(uint32_t dst, const char* src, bool in)
 {
     const int n = in ? BYTES : 0;
     if constexpr (BYTES == 16)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n));
     else
-        asm volatile("cp.async.ca.shared.global [%0], [%1], %3, %2;" ::"r"(dst), "l"(src), "r"(n), "n"(BYTES) : "memory");
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %3, %2;" ::"r"(dst), "l"(src), "r"(n), "n"(BYTES));
 }
 
 // The elements (kk, r) of a ROWS x BK operand slice that thread t copies, each
-// call of f covering a group along the rows
-template <int NT, int E, int ROWS, int BK, typename F>
-__device__ __forceinline__ void for_own(int mode, int t, F&& f)
+// call of f covering a group along the rows: f(at(kk), kk, r). Along the rows
+// a warp takes whole contracted values, its lanes the groups of rows.
+template <int NT, int E, int ROWS, int BK, typename A, typename F>
+__device__ __forceinline__ void for_own(int mode, int t, A&& at, F&& f)
 {
-    if (mode == COPY_VEC || mode == COPY_PAIR) {
-        auto groups = [&](auto n) {
-            constexpr int N = decltype(n)::value, G = ROWS / N;  // groups of N rows
+    constexpr int NW = NT / 32;
+    const int w = t >> 5, lane = t & 31;
+    auto along_rows = [&](auto n) {
+        constexpr int N = decltype(n)::value, G = ROWS / N;  // groups of N rows
+        constexpr int LR = G > 16 ? 32 : G > 8 ? 16 : G > 4 ? 8 : G > 2 ? 4 : 2, KP = 32 / LR;
+        const int lr = lane % LR, lk = lane / LR;
 #pragma unroll
-            for (int u = 0; u < (G * BK + NT - 1) / NT; u++) {
-                const int i = t + NT * u;
-                if (G * BK % NT == 0 || i < G * BK) f(i / G, (i % G) * N);
+        for (int u = 0; u < (BK + NW * KP - 1) / (NW * KP); u++) {
+            const int kk = w * KP + lk + u * NW * KP;
+            if (BK % (NW * KP) && kk >= BK) continue;
+            const int64_t o = at(kk);
+#pragma unroll
+            for (int j = 0; j < (G + LR - 1) / LR; j++) {
+                const int g = lr + j * LR;
+                if (G % LR == 0 || g < G) f(o, kk, g * N);
             }
-        };
-        if (mode == COPY_VEC) groups(std::integral_constant<int, 16 / E>());
-        else groups(std::integral_constant<int, 2>());
-    } else if (mode == COPY_ROWS) {
-#pragma unroll
-        for (int u = 0; u < (ROWS * BK + NT - 1) / NT; u++) {
-            const int i = t + NT * u;
-            if (ROWS * BK % NT == 0 || i < ROWS * BK) f(i / ROWS, i % ROWS);
         }
+    };
+    if (mode == COPY_VEC) {
+        along_rows(std::integral_constant<int, 16 / E>());
+    } else if (E == 4 && mode == COPY_PAIR) {
+        along_rows(std::integral_constant<int, 2>());
+    } else if (mode == COPY_ROWS) {
+        along_rows(std::integral_constant<int, 1>());
     } else {
         // KS lanes along the contraction (32 bytes), RS rows per warp
         constexpr int KS = 32 / E, RS = 32 / KS, KB = BK / KS, UNITS = ROWS * BK / 32;
         static_assert(BK % KS == 0 && ROWS % RS == 0, "whole units of a warp");
-        const int lane = t & 31, kl = lane % KS, rl = lane / KS;
+        const int kl = lane % KS, rl = lane / KS;
 #pragma unroll
-        for (int u = 0; u < (UNITS + NT / 32 - 1) / (NT / 32); u++) {
-            const int q = (t >> 5) + (NT / 32) * u;
-            if (UNITS % (NT / 32) == 0 || q < UNITS) f((q % KB) * KS + kl, (q / KB) * RS + rl);
+        for (int u = 0; u < (UNITS + NW - 1) / NW; u++) {
+            const int q = w + NW * u, kk = (q % KB) * KS + kl;
+            if (UNITS % NW == 0 || q < UNITS) f(at(kk), kk, (q / KB) * RS + rl);
         }
     }
 }
 
-// One slice of an operand: rows < rows_in and kk < k_in exist, the rest is zero
+// One slice of an operand: rows < rows_in and kk < k_in exist, the rest is
+// zero. The tables hold byte offsets, 0 for what does not exist, so that every
+// address lies in the operand.
 template <int NT, int E, int ROWS, int LD, int BK>
 __device__ __forceinline__ void copy_slice(uint32_t dst, const char* base, const int64_t* row, const int64_t* kof,
                                            int rows_in, int k_in, int mode, int half, int t)
 {
-    if (mode == COPY_VEC) {
-        for_own<NT, E, ROWS, BK>(COPY_VEC, t, [&](int kk, int r) {
-            const bool in = r < rows_in && kk < k_in;
-            copy_async<16>(dst + (uint32_t)(kk * LD + r) * E, in ? base + (row[r] + kof[kk]) * E : base, in);
+    auto at = [&](int kk) { return kof[kk]; };
+    auto place = [&](int kk, int r) { return dst + (uint32_t)(kk * LD + r) * E; };
+    if (mode == COPY_VEC)
+        for_own<NT, E, ROWS, BK>(COPY_VEC, t, at, [&](int64_t o, int kk, int r) {
+            copy_async<16>(place(kk, r), base + o + row[r], r < rows_in && kk < k_in);
         });
-        return;
-    }
-    if constexpr (E == 4) {
-        if (mode == COPY_PAIR) {
-            for_own<NT, E, ROWS, BK>(COPY_PAIR, t, [&](int kk, int r) {
-                const bool in = r < rows_in && kk < k_in;
-                copy_async<8>(dst + (uint32_t)(kk * LD + r) * E, in ? base + (row[r] + kof[kk]) * E : base, in);
-            });
-            return;
-        }
-    }
-    auto one = [&](int kk, int r) {
-        const bool in = r < rows_in && kk < k_in;
-        const char* src = in ? base + (row[r] + kof[kk]) * E : base;
-        const uint32_t at = dst + (uint32_t)(kk * LD + r) * E;
-        if constexpr (E >= 8) {
-            if (half) {
-                copy_async<E / 2>(at, src, in);
-                copy_async<E / 2>(at + E / 2, in ? src + E / 2 : src, in);
-                return;
-            }
-        }
-        copy_async<E>(at, src, in);
-    };
-    if (mode == COPY_ROWS) for_own<NT, E, ROWS, BK>(COPY_ROWS, t, one);
-    else for_own<NT, E, ROWS, BK>(COPY_K, t, one);
+    else if (E == 4 && mode == COPY_PAIR)
+        for_own<NT, E, ROWS, BK>(COPY_PAIR, t, at, [&](int64_t o, int kk, int r) {
+            copy_async<8>(place(kk, r), base + o + row[r], r < rows_in && kk < k_in);
+        });
+    else if (E >= 8 && half)  // complex elements aligned to their parts only
+        for_own<NT, E, ROWS, BK>(mode, t, at, [&](int64_t o, int kk, int r) {
+            const bool in = r < rows_in && kk < k_in;
+            copy_async<(E >= 8 ? E / 2 : 4)>(place(kk, r), base + o + row[r], in);
+            copy_async<(E >= 8 ? E / 2 : 4)>(place(kk, r) + E / 2, base + o + row[r] + E / 2, in);
+        });
+    else if (mode == COPY_ROWS)
+        for_own<NT, E, ROWS, BK>(COPY_ROWS, t, at, [&](int64_t o, int kk, int r) {
+            copy_async<E>(place(kk, r), base + o + row[r], r < rows_in && kk < k_in);
+        });
+    else
+        for_own<NT, E, ROWS, BK>(COPY_K, t, at, [&](int64_t o, int kk, int r) {
+            copy_async<E>(place(kk, r), base + o + row[r], r < rows_in && kk < k_in);
+        });
 }
 
 // ---------------------------------------------------------------------------
@@ -667,19 +672,19 @@ __device__ __forceinline__ uint32_t remote(uint32_t at, uint32_t rank)
 }
 __device__ __forceinline__ void load_remote(uint32_t a, float& v)
 {
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a));
 }
 __device__ __forceinline__ void load_remote(uint32_t a, double& v)
 {
-    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(a) : "memory");
+    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(a));
 }
 __device__ __forceinline__ void load_remote(uint32_t a, float2& v)
 {
-    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a) : "memory");
+    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a));
 }
 __device__ __forceinline__ void load_remote(uint32_t a, double2& v)
 {
-    asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(a) : "memory");
+    asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(a));
 }
 
 // RND: binary32 operands rounded to the precision's 16-bit format, by the
@@ -697,10 +702,9 @@ __global__ void __launch_bounds__(W::NT, W::MINB) k_tile(const __grid_constant__
     int64_t* bRow = aRow + BM;
     int64_t* kA = bRow + BN;       // [2][KT]
     int64_t* kB = kA + 2 * KT;
-    int64_t* cRow = kB + 2 * KT;
-    int64_t* dRow = cRow + BM;
-    int64_t* cCol = dRow + BM;
-    int64_t* dCol = cCol + BN;
+    // offsets in C (x) and D (y) of the tile's rows and columns
+    longlong2* rowCD = (longlong2*)(kB + 2 * KT);
+    longlong2* colCD = rowCD + BM;
 
     const int t = threadIdx.x;
     // neighbouring blocks share a row panel of A (the longer operand)
@@ -717,12 +721,12 @@ __global__ void __launch_bounds__(W::NT, W::MINB) k_tile(const __grid_constant__
         const int at = (batch & 1) * KT;
         for (int i = t; i < 2 * KT; i += NT) {
             const int64_t k = k0 + i % KT;
-            if (k < kend) (i < KT ? kA : kB - KT)[at + i] = offset1(i < KT ? p.ak : p.bk, (uint32_t)k);
+            (i < KT ? kA : kB - KT)[at + i] = k < kend ? E * offset1(i < KT ? p.ak : p.bk, (uint32_t)k) : 0;
         }
     };
     for (int i = t; i < BM + BN; i += NT) {
-        if (i < BM) aRow[i] = i < rows_a ? offset1(p.al, l) + offset1(p.am, m0 + i) : 0;
-        else bRow[i - BM] = i - BM < rows_b ? offset1(p.bl, l) + offset1(p.bn, n0 + i - BM) : 0;
+        if (i < BM) aRow[i] = i < rows_a ? E * (offset1(p.al, l) + offset1(p.am, m0 + i)) : 0;
+        else bRow[i - BM] = i - BM < rows_b ? E * (offset1(p.bl, l) + offset1(p.bn, n0 + i - BM)) : 0;
     }
     static_assert(STAGES <= BATCH, "the first slices lie in the first refill");
     fill_offsets(0);
@@ -757,12 +761,10 @@ __global__ void __launch_bounds__(W::NT, W::MINB) k_tile(const __grid_constant__
                         offset2(p.cl, l, lc, ld);
                         offset2(p.cm, m0 + i, oc, od);
                     }
-                    cRow[i] = oc + lc;
-                    dRow[i] = od + ld;
+                    rowCD[i] = make_longlong2(oc + lc, od + ld);
                 } else {
                     if (i - BM < rows_b) offset2(p.cn, n0 + i - BM, oc, od);
-                    cCol[i - BM] = oc;
-                    dCol[i - BM] = od;
+                    colCD[i - BM] = make_longlong2(oc, od);
                 }
             }
         }
@@ -771,7 +773,7 @@ __global__ void __launch_bounds__(W::NT, W::MINB) k_tile(const __grid_constant__
         char* Bs = As + BK * W::LDA * E;
         if (RND && s >= 0) {
             auto round_own = [&](char* base, int ld, int mode) {
-                return [=](int kk, int r) {
+                return [=](int64_t, int kk, int r) {
                     float* x = (float*)base + kk * ld + r;
                     if (mode == COPY_VEC) {
                         float4 v = *(float4*)x;
@@ -790,8 +792,9 @@ __global__ void __launch_bounds__(W::NT, W::MINB) k_tile(const __grid_constant__
                     }
                 };
             };
-            for_own<NT, E, BM, BK>(p.a_copy, t, round_own(As, W::LDA, p.a_copy));
-            for_own<NT, E, BN, BK>(p.b_copy, t, round_own(Bs, W::LDB, p.b_copy));
+            auto none = [](int) { return (int64_t)0; };
+            for_own<NT, E, BM, BK>(p.a_copy, t, none, round_own(As, W::LDA, p.a_copy));
+            for_own<NT, E, BN, BK>(p.b_copy, t, none, round_own(Bs, W::LDB, p.b_copy));
         }
         if (s >= 0) __syncthreads();  // slice s has landed; slice s - 1 has been read by all
         if (s >= 0 && q % BATCH == BATCH / 2 && (q / BATCH + 1) * BATCH < slices) fill_offsets(q / BATCH + 1);
@@ -817,13 +820,14 @@ __global__ void __launch_bounds__(W::NT, W::MINB) k_tile(const __grid_constant__
         const int at = r * sr + c * sc;
         if (ranks == 1) return tile[at];
         const uint32_t a = ring + (uint32_t)(at * (int)sizeof(V));
-        V x, y;
-        load_remote(remote(a, 0), x);
-        for (int z = 1; z < ranks; z++) {
-            load_remote(remote(a, z), y);
-            x = VT::sum(x, y);
-        }
-        return x;
+        V x[8];  // the ranks' loads in flight together
+#pragma unroll
+        for (int z = 0; z < 8; z++)
+            if (z < ranks) load_remote(remote(a, z), x[z]);
+#pragma unroll
+        for (int z = 1; z < 8; z++)
+            if (z < ranks) x[0] = VT::sum(x[0], x[z]);
+        return x[0];
     };
     auto place = [&](int e, int& r, int& c) {
         r = by_rows ? e % BM : e / BN;
@@ -838,42 +842,64 @@ __global__ void __launch_bounds__(W::NT, W::MINB) k_tile(const __grid_constant__
                 ((V*)p.ws)[(((int64_t)blockIdx.y * p.L + l) * p.M + m0 + r) * p.N + n0 + c] = summed(r, c);
         }
     } else if (p.tC == STORED && p.tD == STORED) {
-        // C and D as they are computed: the C values of U outputs loaded
-        // together. (Code for every storage type, unrolled, missed the
-        // instruction cache on each tile.)
-        constexpr int U = sizeof(V) == 4 ? 8 : 4;
-        constexpr int Q = W::CPLX ? 2 : 1;
-        const T *C = (const T*)p.C;
-        T* D = (T*)p.D;
-        for (int e0 = first + t; e0 < first + share; e0 += NT * U) {
-            V x[U];
-            T cr[U], ci[U];
-            int64_t od[U];
-            bool in[U];
+        // C and D as they are computed. A warp takes lines of the tile along
+        // D's contiguous side (32 outputs a step), so the line's offsets are
+        // read once and a lane keeps those of its places: some 12 instructions
+        // an output, where one index decoded per output took 60 and made half
+        // of a small product's time. (And no code per storage type, unrolled:
+        // it missed the instruction cache on each tile.)
+        auto lines = [&](auto rows_fast) {
+            constexpr bool RF = decltype(rows_fast)::value;
+            constexpr int IN = RF ? BM : BN, OUT = RF ? BN : BM, IT = (IN + 31) / 32, NW = NT / 32;
+            constexpr int OU = IT >= 8 || (IT >= 4 && sizeof(V) > 4) ? 1 : (sizeof(V) == 16 ? 4 : 8) / IT;  // lines at a time
+            constexpr int Q = W::CPLX ? 2 : 1;
+            const longlong2* inner = RF ? rowCD : colCD;
+            const longlong2* outer = RF ? colCD : rowCD;
+            const int n_in = RF ? rows_a : rows_b, n_out = RF ? rows_b : rows_a;
+            const int o0 = ranks > 1 ? (int)blockIdx.y * (OUT / ranks) : 0;
+            const int o1 = min(n_out, ranks > 1 ? o0 + OUT / ranks : OUT);
+            const int lane = t & 31;
+            int64_t ic[IT], id[IT];
 #pragma unroll
-            for (int u = 0; u < U; u++) {
-                int r, c;
-                in[u] = place(e0 + NT * u, r, c);
-                cr[u] = ci[u] = 0;
-                if (!in[u]) continue;
-                od[u] = Q * (dRow[r] + dCol[c]);
-                if (!p.beta_zero) {
-                    const int64_t oc = Q * (cRow[r] + cCol[c]);
-                    cr[u] = C[oc];
-                    if (W::CPLX) ci[u] = C[oc + Q - 1];
+            for (int i = 0; i < IT; i++) {
+                const longlong2 q = lane + 32 * i < n_in ? inner[lane + 32 * i] : make_longlong2(0, 0);
+                ic[i] = Q * q.x;
+                id[i] = Q * q.y;
+            }
+#pragma unroll 1
+            for (int o = o0 + (t >> 5); o < o1; o += NW * OU) {
+                T cr[OU][IT], ci[OU][IT];
+#pragma unroll
+                for (int v = 0; v < OU; v++) {
+                    const T* C = (const T*)p.C + Q * (o + v * NW < o1 ? outer[o + v * NW].x : 0);
+#pragma unroll
+                    for (int i = 0; i < IT; i++) {
+                        cr[v][i] = ci[v][i] = 0;
+                        if (p.beta_zero || o + v * NW >= o1 || lane + 32 * i >= n_in) continue;
+                        cr[v][i] = C[ic[i]];
+                        if (W::CPLX) ci[v][i] = C[ic[i] + Q - 1];
+                    }
                 }
-                x[u] = summed(r, c);
-            }
 #pragma unroll
-            for (int u = 0; u < U; u++) {
-                if (!in[u]) continue;
-                if (RND) cr[u] = round_in<T>(cr[u], p.round_in);
-                T vr, vi;
-                simt::epilogue_value<T, W::CPLX, Params>(p, VT::re(x[u]), VT::im(x[u]), cr[u], ci[u], vr, vi);
-                D[od[u]] = vr;
-                if (W::CPLX) D[od[u] + Q - 1] = vi;
+                for (int v = 0; v < OU; v++) {
+                    if (o + v * NW >= o1) break;
+                    T* D = (T*)p.D + Q * outer[o + v * NW].y;
+#pragma unroll
+                    for (int i = 0; i < IT; i++) {
+                        const int at = lane + 32 * i;
+                        if (at >= n_in) continue;
+                        const V x = RF ? summed(at, o + v * NW) : summed(o + v * NW, at);
+                        T c = cr[v][i], vr, vi;
+                        if (RND) c = round_in<T>(c, p.round_in);
+                        simt::epilogue_value<T, W::CPLX, Params>(p, VT::re(x), VT::im(x), c, ci[v][i], vr, vi);
+                        D[id[i]] = vr;
+                        if (W::CPLX) D[id[i] + Q - 1] = vi;
+                    }
+                }
             }
-        }
+        };
+        if (by_rows) lines(std::true_type());
+        else lines(std::false_type());
     } else {
 #pragma unroll 1
         for (int e = first + t; e < first + share; e += NT) {
@@ -881,9 +907,9 @@ __global__ void __launch_bounds__(W::NT, W::MINB) k_tile(const __grid_constant__
             if (!place(e, r, c)) continue;
             const V x = summed(r, c);
             T cr = 0, ci = 0, vr, vi;
-            if (!p.beta_zero) load_rounded<T>(p.C, cRow[r] + cCol[c], p.tC, p.round_in, cr, ci);
+            if (!p.beta_zero) load_rounded<T>(p.C, rowCD[r].x + colCD[c].x, p.tC, p.round_in, cr, ci);
             simt::epilogue_value<T, W::CPLX, Params>(p, VT::re(x), VT::im(x), cr, ci, vr, vi);
-            store_elem<T>(p.D, dRow[r] + dCol[c], p.tD, vr, vi);
+            store_elem<T>(p.D, rowCD[r].y + colCD[c].y, p.tD, vr, vi);
         }
     }
     if (ranks > 1) cluster_barrier();  // no block leaves while its tile may be read
