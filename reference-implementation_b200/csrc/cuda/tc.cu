@@ -297,34 +297,19 @@ __global__ void __launch_bounds__(256, 4) k_pack_real(PackParams p)
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
-// Pipelined pack for binary32 sources contiguous along the contraction and
-// read 16 bytes at a time (the VEC = 4, K-fast case above: the first
-// contracted mode has stride 1 and an extent divisible by 4, every other
-// stride keeps 16-byte alignment). Persistent blocks of 128 threads walk the
-// 64 x 64 tiles (block b: tiles b, b + grid, ...) and copy each tile into a
-// ring of PP_STAGES shared-memory slots with cp.async, PP_STAGES - 1 tiles
-// ahead of the one being written out, so a block keeps ~48 KiB of loads in
-// flight without holding them in registers (the one-tile kernel above has one
-// load phase and one store phase per block). Slot layout [r][k], 68 floats
-// per row, read without bank conflicts: thread (r, g) reads k = 8g..8g+7 as
-// two 16-byte reads, lanes 4-7 of each quarter-warp reading their second half
-// first. Output words and their order are those of k_pack_real (same
-// rounding, same [hi | lo] or three-segment split), so the two kernels write
-// identical panels. On the 64^4 contraction's B operand: 23.2 us against
-// 26.9 us for k_pack_real; for sources contiguous along the rows the
-// transposed reads made it slower than k_pack_real (41.8 against 28.0 us),
-// so those keep k_pack_real.
-constexpr int PP_THREADS = 128, PP_STAGES = 4, PP_PITCH = 68;
-constexpr int PP_SLOT = 64 * PP_PITCH;  // floats per slot
-struct PackTab {
-    int64_t row[64];
-    int64_t k[64];
-    const float* src;  // the tile's batch base
-    int64_t pad;
-};
-constexpr int PP_SMEM = PP_STAGES * PP_SLOT * 4 + 2 * (int)sizeof(PackTab);
+// Pack of binary32 sources contiguous along the contraction and read 16 bytes
+// at a time (the VEC = 4, K-fast case above: the first contracted mode has
+// stride 1 and an extent divisible by 4, every other stride keeps 16-byte
+// alignment). Source and panel run the same way, so nothing is staged: a warp
+// takes a row's 256 contracted values, a lane 8 of them (two 16-byte reads,
+// one 16-byte write per segment), and a thread has the reads of 4 rows in
+// flight. Output words and their order are those of k_pack_real (same
+// rounding, same segments), so the two kernels write identical panels.
+// On the 64^4 contraction's B operand 17.4 us (5.5 TB/s) against 25.5 us through
+// a ring of shared-memory tiles, [hi | lo] 21 against 24 us.
+constexpr int PR_ROWS = 32, PR_K = 256, PR_THREADS = 256;
 
-// multiply-high divisors of the pipelined pack's index arithmetic (every
+// multiply-high divisors of that pack's index arithmetic (every
 // extent, row count, contraction length and tile count below 2^31)
 struct PackDivs {
     FastDiv rows[TB_MAXMODES], ks[TB_MAXMODES], ls[TB_MAXMODES];
@@ -341,15 +326,6 @@ __device__ __forceinline__ int64_t pp_decode(const ModeList& m, const FastDiv* f
     }
     return o;
 }
-
-__device__ __forceinline__ void cp_async16_zfill(uint32_t dst, const void* src, bool in)
-{
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16 : 0)
-                 : "memory");
-}
-__device__ __forceinline__ void pp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void pp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 // eight values of row rg at columns col..col+7, every segment, as k_pack_real writes them
 template <int SPLIT, int FMT>
@@ -385,94 +361,50 @@ __device__ __forceinline__ void pp_put8(const PackParams& p, int64_t l, int64_t 
 }
 
 template <int SPLIT, int FMT>
-__global__ void __launch_bounds__(PP_THREADS) k_pack_pipe(PackParams p, PackDivs dv, int32_t ntiles)
+__global__ void __launch_bounds__(PR_THREADS) k_pack_runs(PackParams p, PackDivs dv)
 {
     // a GEMM launched after this pack as a programmatic dependent may start
     // its set-up once every block of this grid has begun; it reads nothing
     // of the panels before this grid has finished (griddepcontrol.wait)
     asm volatile("griddepcontrol.launch_dependents;");
-    extern __shared__ __align__(16) float pp_sm[];
-    float* slots = pp_sm;
-    PackTab* tab = (PackTab*)(pp_sm + PP_STAGES * PP_SLOT);
+    __shared__ int64_t row[PR_ROWS], run[PR_K / 4];
+    __shared__ const float* base;
     const int t = threadIdx.x;
-    const int32_t first = blockIdx.x, step = gridDim.x;
-    const int32_t nloc = first < ntiles ? (ntiles - 1 - first) / step + 1 : 0;
-    auto tile_of = [&](int32_t i, int64_t& r0, int64_t& k0, int64_t& l) {
-        const uint32_t j = (uint32_t)(first + i * step);
-        const uint32_t jk = fdiv(j, dv.tiles_k), jr = fdiv(jk, dv.tiles_r);
-        k0 = (int64_t)(j - jk * dv.tiles_k.d) * 64;
-        r0 = (int64_t)(jk - jr * dv.tiles_r.d) * 64;
-        l = jr;
-    };
-    // source offsets of tile i's 64 rows (threads 0-63) and 64 columns (64-127)
-    auto make_tab = [&](int32_t i, PackTab& tb) {
-        if (i >= nloc) return;
-        int64_t r0, k0, l, o = 0;
-        tile_of(i, r0, k0, l);
-        if (t < 64) {
-            if (r0 + t < p.R) o = pp_decode(p.rows, dv.rows, (uint32_t)(r0 + t));
-            tb.row[t] = o;
-        } else {
-            const int kk = t - 64;
-            if (k0 + kk < p.K) o = pp_decode(p.ks, dv.ks, (uint32_t)(k0 + kk));
-            tb.k[kk] = o;
-        }
-        if (t == 0) {
-            const uint32_t b = p.srcs ? fdiv((uint32_t)l, dv.lsz) : 0u;
-            const uint32_t lsrc = (uint32_t)l - b * dv.lsz.d;
-            o = pp_decode(p.ls, dv.ls, p.srcs ? lsrc : (uint32_t)l);
-            tb.src = (const float*)(p.srcs ? p.srcs[b] : p.src) + o;
-        }
-    };
-    // 1024 chunks of 16 bytes per tile, 8 per thread; outside the tensor: zeros
-    auto issue = [&](int32_t i, const PackTab& tb) {
-        if (i < nloc) {
-            int64_t r0, k0, l;
-            tile_of(i, r0, k0, l);
-            const uint32_t sb = smem_u32(slots + (i % PP_STAGES) * PP_SLOT);
-#pragma unroll
-            for (int u = 0; u < 8; u++) {
-                const int c = t + PP_THREADS * u;
-                const int r = c / 16, kk = (c % 16) * 4;
-                const uint32_t dst = sb + (uint32_t)(r * PP_PITCH + kk) * 4u;
-                const bool in = r0 + r < p.R && k0 + kk < p.K;
-                cp_async16_zfill(dst, in ? (const void*)(tb.src + tb.row[r] + tb.k[kk]) : (const void*)tb.src, in);
-            }
-        }
-        pp_commit();  // empty groups keep the count uniform
-    };
-    auto store = [&](int32_t i) {
-        int64_t r0, k0, l;
-        tile_of(i, r0, k0, l);
-        const float* v = slots + (i % PP_STAGES) * PP_SLOT;
-#pragma unroll
-        for (int it = 0; it < 4; it++) {
-            const int e = t + PP_THREADS * it;
-            const int g = e % 8, r = e / 8;
-            const int64_t rg = r0 + r, col = k0 + g * 8;
-            if (rg >= p.R || col >= p.Kseg) continue;
-            const int h0 = (g >> 2) & 1;
-            const float4 a = *(const float4*)(v + r * PP_PITCH + g * 8 + 4 * h0);
-            const float4 b = *(const float4*)(v + r * PP_PITCH + g * 8 + 4 * (1 - h0));
-            const float4 lo4 = h0 ? b : a, hi4 = h0 ? a : b;
-            const float x[8] = {lo4.x, lo4.y, lo4.z, lo4.w, hi4.x, hi4.y, hi4.z, hi4.w};
-            pp_put8<SPLIT, FMT>(p, l, rg, col, x);
-        }
-    };
-    for (int i = 0; i < PP_STAGES - 1; i++) {
-        make_tab(i, tab[i & 1]);
-        __syncthreads();
-        issue(i, tab[i & 1]);
+    const uint32_t jk = fdiv(blockIdx.x, dv.tiles_k), jr = fdiv(jk, dv.tiles_r);
+    const int64_t k0 = (int64_t)(blockIdx.x - jk * dv.tiles_k.d) * PR_K, r0 = (int64_t)(jk - jr * dv.tiles_r.d) * PR_ROWS;
+    const int64_t l = jr;
+    if (t < PR_ROWS) {
+        row[t] = r0 + t < p.R ? pp_decode(p.rows, dv.rows, (uint32_t)(r0 + t)) : 0;
+    } else if (t < PR_ROWS + PR_K / 4) {
+        const int64_t k = k0 + (t - PR_ROWS) * 4;
+        run[t - PR_ROWS] = k < p.K ? pp_decode(p.ks, dv.ks, (uint32_t)k) : 0;
+    } else if (t == PR_ROWS + PR_K / 4) {
+        const uint32_t b = p.srcs ? fdiv((uint32_t)l, dv.lsz) : 0u;
+        const uint32_t lsrc = (uint32_t)l - b * dv.lsz.d;
+        base = (const float*)(p.srcs ? p.srcs[b] : p.src) + pp_decode(p.ls, dv.ls, p.srcs ? lsrc : (uint32_t)l);
     }
-    make_tab(PP_STAGES - 1, tab[(PP_STAGES - 1) & 1]);
-    for (int32_t i = 0; i < nloc; i++) {
-        pp_wait<PP_STAGES - 2>();  // this thread's copies of tile i have landed
-        __syncthreads();           // everyone's have; slot (i - 1) and table (i + S) are free
-        issue(i + PP_STAGES - 1, tab[(i + PP_STAGES - 1) & 1]);
-        make_tab(i + PP_STAGES, tab[(i + PP_STAGES) & 1]);
-        store(i);
+    __syncthreads();
+    constexpr int U = PR_ROWS * 32 / PR_THREADS;  // rows of a thread
+    const int g = t % 32, r = t / 32;
+    const int64_t col = k0 + g * 8;
+    const float *lo = base + run[2 * g], *hi = base + run[2 * g + 1];
+    const bool lo_in = col < p.K, hi_in = col + 4 < p.K;
+    float4 a[U], b[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        const int i = r + u * (PR_THREADS / 32);
+        const bool in = r0 + i < p.R;
+        a[u] = b[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (in && lo_in) a[u] = __ldg((const float4*)(lo + row[i]));
+        if (in && hi_in) b[u] = __ldg((const float4*)(hi + row[i]));
     }
-    pp_wait<0>();
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        const int64_t rg = r0 + r + u * (PR_THREADS / 32);
+        if (rg >= p.R || col >= p.Kseg) continue;
+        const float x[8] = {a[u].x, a[u].y, a[u].z, a[u].w, b[u].x, b[u].y, b[u].z, b[u].w};
+        pp_put8<SPLIT, FMT>(p, l, rg, col, x);
+    }
     // launched as a programmatic dependent of the pack before it (the first
     // operand's), this grid ends only after that one has: whoever waits for
     // this grid's completion then has both operands' panels
@@ -502,24 +434,10 @@ static void launch_pack_kernel(K kern, dim3 grid, unsigned threads, size_t smem,
     (void)cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
-// false: the kernel could not be given its shared memory (the caller runs k_pack_real)
 template <int SPLIT, int FMT>
-static bool launch_pack_pipe(const PackParams& pp, int64_t lz, cudaStream_t s, bool pdl)
+static void launch_pack_runs(const PackParams& pp, int64_t lz, cudaStream_t s, bool pdl)
 {
-    auto kern = k_pack_pipe<SPLIT, FMT>;
-    static int attr_done[64];
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64 || !attr_done[dev]) {
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PP_SMEM) != cudaSuccess) {
-            cudaGetLastError();
-            return false;
-        }
-        if (dev >= 0 && dev < 64) attr_done[dev] = 1;
-    }
-    const int64_t tiles_r = (pp.R + 63) / 64, tiles_k = (pp.Kseg + 63) / 64;
-    const int64_t ntiles = tiles_r * tiles_k * lz;
-    const int64_t grid = std::min<int64_t>(ntiles, (int64_t)num_sms() * 3);
+    const int64_t tiles_r = (pp.R + PR_ROWS - 1) / PR_ROWS, tiles_k = (pp.Kseg + PR_K - 1) / PR_K;
     PackDivs dv;
     memset(&dv, 0, sizeof(dv));
     for (int j = 0; j < pp.rows.n; j++) dv.rows[j] = make_fastdiv((uint32_t)pp.rows.ext[j]);
@@ -528,15 +446,15 @@ static bool launch_pack_pipe(const PackParams& pp, int64_t lz, cudaStream_t s, b
     dv.tiles_k = make_fastdiv((uint32_t)tiles_k);
     dv.tiles_r = make_fastdiv((uint32_t)tiles_r);
     dv.lsz = make_fastdiv((uint32_t)std::max<int64_t>(pp.Lsz, 1));
-    if (grid > 0) launch_pack_kernel(kern, dim3((unsigned)grid), PP_THREADS, PP_SMEM, s, pdl, pp, dv, (int32_t)ntiles);
-    return true;
+    const int64_t grid = tiles_r * tiles_k * lz;
+    if (grid > 0) launch_pack_kernel(k_pack_runs<SPLIT, FMT>, dim3((unsigned)grid), PR_THREADS, 0, s, pdl, pp, dv);
 }
 
-// the pipelined pack's 32-bit index arithmetic covers the operand
-static bool pack_pipe_fits(const PackParams& pp, int64_t lz)
+// that pack's 32-bit index arithmetic covers the operand
+static bool pack_runs_fits(const PackParams& pp, int64_t lz)
 {
     const int64_t lim = (int64_t)1 << 31;
-    const int64_t ntiles = ((pp.R + 63) / 64) * ((pp.Kseg + 63) / 64) * lz;
+    const int64_t ntiles = ((pp.R + PR_ROWS - 1) / PR_ROWS) * ((pp.Kseg + PR_K - 1) / PR_K) * lz;
     if (pp.R >= lim || pp.Kseg >= lim || pp.K >= lim || lz >= lim || ntiles >= lim) return false;
     const ModeList* ms[3] = {&pp.rows, &pp.ks, &pp.ls};
     for (const ModeList* m : ms)
@@ -545,12 +463,12 @@ static bool pack_pipe_fits(const PackParams& pp, int64_t lz)
     return !pp.srcs || pp.Lsz >= 1;
 }
 
-static bool launch_pack_pipe3(const PackParams& pp, int split, int fmt, int64_t lz, cudaStream_t s, bool pdl)
+static void launch_pack_runs3(const PackParams& pp, int split, int fmt, int64_t lz, cudaStream_t s, bool pdl)
 {
-    if (split == 3) return launch_pack_pipe<3, 0>(pp, lz, s, pdl);
-    if (split == 2) return launch_pack_pipe<2, 0>(pp, lz, s, pdl);
-    if (fmt == 1) return launch_pack_pipe<1, 1>(pp, lz, s, pdl);
-    return launch_pack_pipe<1, 0>(pp, lz, s, pdl);
+    if (split == 3) launch_pack_runs<3, 0>(pp, lz, s, pdl);
+    else if (split == 2) launch_pack_runs<2, 0>(pp, lz, s, pdl);
+    else if (fmt == 1) launch_pack_runs<1, 1>(pp, lz, s, pdl);
+    else launch_pack_runs<1, 0>(pp, lz, s, pdl);
 }
 
 template <typename T, bool RF, int VEC>
@@ -588,7 +506,10 @@ static void launch_pack_real(const PackParams& pp, int split, int fmt, int64_t l
         const ModeList* others[3] = {rf ? &pp.ks : &pp.rows, &pp.ls, &pp.us};
         v4 = vec4_ok(rf ? pp.rows : pp.ks, others, 2, pp.src);
     }
-    if (v4 && !rf && pack_pipe_fits(pp, lz) && launch_pack_pipe3(pp, split, fmt, lz, s, pdl)) return;
+    if (v4 && !rf && pack_runs_fits(pp, lz)) {
+        launch_pack_runs3(pp, split, fmt, lz, s, pdl);
+        return;
+    }
     if (rf) {
         if (v4) launch_pack_real3<T, true, 4>(pp, split, fmt, grid, s, pdl);
         else launch_pack_real3<T, true, 1>(pp, split, fmt, grid, s, pdl);
