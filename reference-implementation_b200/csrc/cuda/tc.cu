@@ -196,10 +196,9 @@ __device__ __forceinline__ float load_as_float<__nv_bfloat16>(const void* base, 
 }
 
 // ROWS_FAST: the source is contiguous along the first row (M or N) mode, else
-// along the first contracted mode. VEC = 4: that mode has stride 1, an extent
-// divisible by 4 and every other stride (and the base) keeps 16-byte
-// alignment, so four neighbours come in one 16-byte load.
-template <typename T, int SPLIT, int FMT, bool ROWS_FAST, int VEC>
+// along the first contracted mode. Binary32 sources in 16-byte groups go to
+// k_pack_runs and k_pack_cols below.
+template <typename T, int SPLIT, int FMT, bool ROWS_FAST>
 __global__ void __launch_bounds__(256, 4) k_pack_real(PackParams p)
 {
     // a GEMM launched after this pack as a programmatic dependent may start
@@ -228,37 +227,25 @@ __global__ void __launch_bounds__(256, 4) k_pack_real(PackParams p)
         lOff = o;
     }
     __syncthreads();
-    constexpr int NV = FR * FK / 256 / VEC;  // vector loads per thread
-    constexpr int G = (ROWS_FAST ? FR : FK) / VEC;  // vectors along the fast direction
-    float x[NV][VEC];
+    constexpr int NV = FR * FK / 256;  // loads per thread
+    constexpr int G = ROWS_FAST ? FR : FK;
+    float x[NV];
 #pragma unroll
     for (int u = 0; u < NV; u++) {
         const int e = t + 256 * u;
-        const int fg = e % G, sl = e / G;              // fast-direction group, slow index
-        const int r = ROWS_FAST ? fg * VEC : sl;
-        const int kk = ROWS_FAST ? sl : fg * VEC;
+        const int fast = e % G, slow = e / G;
+        const int r = ROWS_FAST ? fast : slow;
+        const int kk = ROWS_FAST ? slow : fast;
         const bool in = (r0 + r < p.R) && (k0 + kk < p.K);
-        const int64_t off = lOff + rowOff[r] + kOff[kk];
-        if (VEC == 4) {
-            float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (in) q = __ldg((const float4*)((const float*)src + off));
-            x[u][0] = q.x; x[u][VEC > 1 ? 1 : 0] = q.y; x[u][VEC > 2 ? 2 : 0] = q.z; x[u][VEC > 3 ? 3 : 0] = q.w;
-        } else {
-            x[u][0] = in ? load_as_float<T>(src, off) : 0.f;
-        }
+        x[u] = in ? load_as_float<T>(src, lOff + rowOff[r] + kOff[kk]) : 0.f;
     }
 #pragma unroll
     for (int u = 0; u < NV; u++) {
         const int e = t + 256 * u;
-        const int fg = e % G, sl = e / G;
-#pragma unroll
-        for (int h = 0; h < VEC; h++) {
-            const int r = ROWS_FAST ? fg * VEC + h : sl;
-            const int kk = ROWS_FAST ? sl : fg * VEC + h;
-            float y = x[u][h];
-            if (SPLIT == 1 && p.round_mode != TB_ROUND_NONE) y = round_in<float>(y, p.round_mode);
-            v[r][kk] = y;
-        }
+        const int fast = e % G, slow = e / G;
+        float y = x[u];
+        if (SPLIT == 1 && p.round_mode != TB_ROUND_NONE) y = round_in<float>(y, p.round_mode);
+        v[ROWS_FAST ? fast : slow][ROWS_FAST ? slow : fast] = y;
     }
     __syncthreads();
     // FR rows x FK/8 groups of eight per segment
@@ -297,19 +284,27 @@ __global__ void __launch_bounds__(256, 4) k_pack_real(PackParams p)
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
-// Pack of binary32 sources contiguous along the contraction and read 16 bytes
-// at a time (the VEC = 4, K-fast case above: the first contracted mode has
-// stride 1 and an extent divisible by 4, every other stride keeps 16-byte
-// alignment). Source and panel run the same way, so nothing is staged: a warp
+// Packs of binary32 sources read 16 bytes at a time: the contiguous mode (the
+// first contracted or the first row mode) has stride 1 and an extent divisible
+// by 4, every other stride and the base keep 16-byte alignment.
+//
+// k_pack_runs, contiguous along the contraction: source and panel run the same way, so nothing is staged: a warp
 // takes a row's 256 contracted values, a lane 8 of them (two 16-byte reads,
 // one 16-byte write per segment), and a thread has the reads of 4 rows in
 // flight. Output words and their order are those of k_pack_real (same
 // rounding, same segments), so the two kernels write identical panels.
 // On the 64^4 contraction's B operand 17.4 us (5.5 TB/s) against 25.5 us through
 // a ring of shared-memory tiles, [hi | lo] 21 against 24 us.
-constexpr int PR_ROWS = 32, PR_K = 256, PR_THREADS = 256;
+//
+// k_pack_cols, contiguous along the rows: a lane reads 4 rows of 8 contracted
+// values (8 reads of 16 bytes in flight) and writes 8 values of each row,
+// transposed in registers; a warp's 4 x 8 lanes cover 16 rows x 64 values, so
+// that it reads runs of 64 and writes runs of 128 bytes (8 x 4 lanes, the other
+// way round, wrote [hi | lo] in 29 us). On the 64^4 contraction's A 18.9 us
+// (5.1 TB/s) against 22.4 us through shared memory, [hi | lo] 23.1 against 27.8 us.
+constexpr int PR_ROWS = 32, PR_K = 256, PC_ROWS = 64, PC_K = 128, PR_THREADS = 256;
 
-// multiply-high divisors of that pack's index arithmetic (every
+// multiply-high divisors of those packs' index arithmetic (every
 // extent, row count, contraction length and tile count below 2^31)
 struct PackDivs {
     FastDiv rows[TB_MAXMODES], ks[TB_MAXMODES], ls[TB_MAXMODES];
@@ -411,6 +406,50 @@ __global__ void __launch_bounds__(PR_THREADS) k_pack_runs(PackParams p, PackDivs
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+template <int SPLIT, int FMT>
+__global__ void __launch_bounds__(PR_THREADS) k_pack_cols(PackParams p, PackDivs dv)
+{
+    asm volatile("griddepcontrol.launch_dependents;");  // as in k_pack_runs
+    __shared__ int64_t quad[PC_ROWS / 4], kof[PC_K];
+    __shared__ const float* base;
+    const int t = threadIdx.x;
+    const uint32_t jk = fdiv(blockIdx.x, dv.tiles_k), jr = fdiv(jk, dv.tiles_r);
+    const int64_t k0 = (int64_t)(blockIdx.x - jk * dv.tiles_k.d) * PC_K, r0 = (int64_t)(jk - jr * dv.tiles_r.d) * PC_ROWS;
+    const int64_t l = jr;
+    if (t < PC_K) {
+        kof[t] = k0 + t < p.K ? pp_decode(p.ks, dv.ks, (uint32_t)(k0 + t)) : 0;
+    } else if (t < PC_K + PC_ROWS / 4) {
+        const int64_t r = r0 + (t - PC_K) * 4;
+        quad[t - PC_K] = r < p.R ? pp_decode(p.rows, dv.rows, (uint32_t)r) : 0;
+    } else if (t == PC_K + PC_ROWS / 4) {
+        const uint32_t b = p.srcs ? fdiv((uint32_t)l, dv.lsz) : 0u;
+        const uint32_t lsrc = (uint32_t)l - b * dv.lsz.d;
+        base = (const float*)(p.srcs ? p.srcs[b] : p.src) + pp_decode(p.ls, dv.ls, p.srcs ? lsrc : (uint32_t)l);
+    }
+    __syncthreads();
+    const int w = t / 32, lane = t % 32;
+    const int r = w % 4 * 16 + lane % 4 * 4, k = w / 4 * 64 + lane / 4 * 8;
+    const float* src = base + quad[r / 4];
+    const bool row_in = r0 + r < p.R;
+    float4 v[8];
+#pragma unroll
+    for (int u = 0; u < 8; u++) {
+        v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (row_in && k0 + k + u < p.K) v[u] = __ldg((const float4*)(src + kof[k + u]));
+    }
+    if (row_in && k0 + k < p.Kseg) {
+        const float x0[8] = {v[0].x, v[1].x, v[2].x, v[3].x, v[4].x, v[5].x, v[6].x, v[7].x};
+        const float x1[8] = {v[0].y, v[1].y, v[2].y, v[3].y, v[4].y, v[5].y, v[6].y, v[7].y};
+        const float x2[8] = {v[0].z, v[1].z, v[2].z, v[3].z, v[4].z, v[5].z, v[6].z, v[7].z};
+        const float x3[8] = {v[0].w, v[1].w, v[2].w, v[3].w, v[4].w, v[5].w, v[6].w, v[7].w};
+        pp_put8<SPLIT, FMT>(p, l, r0 + r, k0 + k, x0);
+        pp_put8<SPLIT, FMT>(p, l, r0 + r + 1, k0 + k, x1);
+        pp_put8<SPLIT, FMT>(p, l, r0 + r + 2, k0 + k, x2);
+        pp_put8<SPLIT, FMT>(p, l, r0 + r + 3, k0 + k, x3);
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // as in k_pack_runs
+}
+
 static int num_sms();
 
 // Launches a pack kernel; pdl: as a programmatic dependent of the pack just
@@ -435,9 +474,11 @@ static void launch_pack_kernel(K kern, dim3 grid, unsigned threads, size_t smem,
 }
 
 template <int SPLIT, int FMT>
-static void launch_pack_runs(const PackParams& pp, int64_t lz, cudaStream_t s, bool pdl)
+static void launch_pack_vec(const PackParams& pp, int64_t lz, cudaStream_t s, bool pdl)
 {
-    const int64_t tiles_r = (pp.R + PR_ROWS - 1) / PR_ROWS, tiles_k = (pp.Kseg + PR_K - 1) / PR_K;
+    const bool rf = pp.rows_fast != 0;
+    const int64_t tr = rf ? PC_ROWS : PR_ROWS, tk = rf ? PC_K : PR_K;
+    const int64_t tiles_r = (pp.R + tr - 1) / tr, tiles_k = (pp.Kseg + tk - 1) / tk;
     PackDivs dv;
     memset(&dv, 0, sizeof(dv));
     for (int j = 0; j < pp.rows.n; j++) dv.rows[j] = make_fastdiv((uint32_t)pp.rows.ext[j]);
@@ -447,14 +488,16 @@ static void launch_pack_runs(const PackParams& pp, int64_t lz, cudaStream_t s, b
     dv.tiles_r = make_fastdiv((uint32_t)tiles_r);
     dv.lsz = make_fastdiv((uint32_t)std::max<int64_t>(pp.Lsz, 1));
     const int64_t grid = tiles_r * tiles_k * lz;
-    if (grid > 0) launch_pack_kernel(k_pack_runs<SPLIT, FMT>, dim3((unsigned)grid), PR_THREADS, 0, s, pdl, pp, dv);
+    if (grid > 0)
+        launch_pack_kernel(rf ? k_pack_cols<SPLIT, FMT> : k_pack_runs<SPLIT, FMT>, dim3((unsigned)grid), PR_THREADS, 0, s, pdl,
+                           pp, dv);
 }
 
-// that pack's 32-bit index arithmetic covers the operand
-static bool pack_runs_fits(const PackParams& pp, int64_t lz)
+// those packs' 32-bit index arithmetic covers the operand
+static bool pack_vec_fits(const PackParams& pp, int64_t lz)
 {
     const int64_t lim = (int64_t)1 << 31;
-    const int64_t ntiles = ((pp.R + PR_ROWS - 1) / PR_ROWS) * ((pp.Kseg + PR_K - 1) / PR_K) * lz;
+    const int64_t ntiles = ((pp.R + PR_ROWS - 1) / PR_ROWS) * ((pp.Kseg + PC_K - 1) / PC_K) * lz;  // at most
     if (pp.R >= lim || pp.Kseg >= lim || pp.K >= lim || lz >= lim || ntiles >= lim) return false;
     const ModeList* ms[3] = {&pp.rows, &pp.ks, &pp.ls};
     for (const ModeList* m : ms)
@@ -463,21 +506,21 @@ static bool pack_runs_fits(const PackParams& pp, int64_t lz)
     return !pp.srcs || pp.Lsz >= 1;
 }
 
-static void launch_pack_runs3(const PackParams& pp, int split, int fmt, int64_t lz, cudaStream_t s, bool pdl)
+static void launch_pack_vec3(const PackParams& pp, int split, int fmt, int64_t lz, cudaStream_t s, bool pdl)
 {
-    if (split == 3) launch_pack_runs<3, 0>(pp, lz, s, pdl);
-    else if (split == 2) launch_pack_runs<2, 0>(pp, lz, s, pdl);
-    else if (fmt == 1) launch_pack_runs<1, 1>(pp, lz, s, pdl);
-    else launch_pack_runs<1, 0>(pp, lz, s, pdl);
+    if (split == 3) launch_pack_vec<3, 0>(pp, lz, s, pdl);
+    else if (split == 2) launch_pack_vec<2, 0>(pp, lz, s, pdl);
+    else if (fmt == 1) launch_pack_vec<1, 1>(pp, lz, s, pdl);
+    else launch_pack_vec<1, 0>(pp, lz, s, pdl);
 }
 
-template <typename T, bool RF, int VEC>
+template <typename T, bool RF>
 static void launch_pack_real3(const PackParams& pp, int split, int fmt, dim3 grid, cudaStream_t s, bool pdl)
 {
-    if (split == 3) launch_pack_kernel(k_pack_real<T, 3, 0, RF, VEC>, grid, 256, 0, s, pdl, pp);
-    else if (split == 2) launch_pack_kernel(k_pack_real<T, 2, 0, RF, VEC>, grid, 256, 0, s, pdl, pp);
-    else if (fmt == 1) launch_pack_kernel(k_pack_real<T, 1, 1, RF, VEC>, grid, 256, 0, s, pdl, pp);
-    else launch_pack_kernel(k_pack_real<T, 1, 0, RF, VEC>, grid, 256, 0, s, pdl, pp);
+    if (split == 3) launch_pack_kernel(k_pack_real<T, 3, 0, RF>, grid, 256, 0, s, pdl, pp);
+    else if (split == 2) launch_pack_kernel(k_pack_real<T, 2, 0, RF>, grid, 256, 0, s, pdl, pp);
+    else if (fmt == 1) launch_pack_kernel(k_pack_real<T, 1, 1, RF>, grid, 256, 0, s, pdl, pp);
+    else launch_pack_kernel(k_pack_real<T, 1, 0, RF>, grid, 256, 0, s, pdl, pp);
 }
 
 // whether a mode list's first mode has stride 1 and extent % 4 == 0 and all
@@ -506,17 +549,9 @@ static void launch_pack_real(const PackParams& pp, int split, int fmt, int64_t l
         const ModeList* others[3] = {rf ? &pp.ks : &pp.rows, &pp.ls, &pp.us};
         v4 = vec4_ok(rf ? pp.rows : pp.ks, others, 2, pp.src);
     }
-    if (v4 && !rf && pack_runs_fits(pp, lz)) {
-        launch_pack_runs3(pp, split, fmt, lz, s, pdl);
-        return;
-    }
-    if (rf) {
-        if (v4) launch_pack_real3<T, true, 4>(pp, split, fmt, grid, s, pdl);
-        else launch_pack_real3<T, true, 1>(pp, split, fmt, grid, s, pdl);
-    } else {
-        if (v4) launch_pack_real3<T, false, 4>(pp, split, fmt, grid, s, pdl);
-        else launch_pack_real3<T, false, 1>(pp, split, fmt, grid, s, pdl);
-    }
+    if (v4 && pack_vec_fits(pp, lz)) launch_pack_vec3(pp, split, fmt, lz, s, pdl);
+    else if (rf) launch_pack_real3<T, true>(pp, split, fmt, grid, s, pdl);
+    else launch_pack_real3<T, false>(pp, split, fmt, grid, s, pdl);
 }
 
 // Self-test of the bounded waits: one thread waits, with the kernels' own
