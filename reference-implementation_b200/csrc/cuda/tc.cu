@@ -229,23 +229,22 @@ __global__ void __launch_bounds__(256, 4) k_pack_real(PackParams p)
     __syncthreads();
     constexpr int NV = FR * FK / 256;  // loads per thread
     constexpr int G = ROWS_FAST ? FR : FK;
+    // the thread's elements: the same fast index, every 256 / G-th slow one
+    const int fast = t % G, slow = t / G;
     float x[NV];
 #pragma unroll
     for (int u = 0; u < NV; u++) {
-        const int e = t + 256 * u;
-        const int fast = e % G, slow = e / G;
-        const int r = ROWS_FAST ? fast : slow;
-        const int kk = ROWS_FAST ? slow : fast;
+        const int r = ROWS_FAST ? fast : slow + 256 / G * u;
+        const int kk = ROWS_FAST ? slow + 256 / G * u : fast;
         const bool in = (r0 + r < p.R) && (k0 + kk < p.K);
-        x[u] = in ? load_as_float<T>(src, lOff + rowOff[r] + kOff[kk]) : 0.f;
+        const int64_t off = lOff + rowOff[r] + kOff[kk];
+        x[u] = in ? load_as_float<T>(src, off) : 0.f;
     }
 #pragma unroll
     for (int u = 0; u < NV; u++) {
-        const int e = t + 256 * u;
-        const int fast = e % G, slow = e / G;
         float y = x[u];
         if (SPLIT == 1 && p.round_mode != TB_ROUND_NONE) y = round_in<float>(y, p.round_mode);
-        v[ROWS_FAST ? fast : slow][ROWS_FAST ? slow : fast] = y;
+        v[ROWS_FAST ? fast : slow + 256 / G * u][ROWS_FAST ? slow + 256 / G * u : fast] = y;
     }
     __syncthreads();
     // FR rows x FK/8 groups of eight per segment
