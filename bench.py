@@ -565,7 +565,7 @@ def element_measure(lib, torch, steps=20, warmup=3):
                 outputs are walked in A's stride order;
       matvec    batched matrix-vector D[m,h] = sum_k A[k,m,h] B[k,h] + C,
                 k = 300, m = 2000, h = 64, A contiguous along k: one warp per
-                output (k_warpdot);
+                output (k_warp_rows);
       c2        the mixed-class complex product (element kernel)."""
     from tapp_b200.workloads import RequestSpec, case_from_spec, mixed_classes_case
     stream = torch.cuda.current_stream().cuda_stream
