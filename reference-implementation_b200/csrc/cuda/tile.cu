@@ -1210,8 +1210,8 @@ bool tile_over_narrow(const simt::Params& p, int compute, int kind)
 {
     if (!tile_takes(p, compute)) return false;
     const double rows = (double)p.M * (double)p.L;
-    if (compute == TB_R64) return p.K >= 64;
     const bool vectors = kind >= 5;
+    if (compute == TB_R64) return vectors ? p.K >= 64 : p.K > 64;
     if (vectors) return p.K > 130 && rows < 148.0 * 256;
     return p.K > 64 && (compute == TB_C32 || rows < 148.0 * 1024);
 }
