@@ -51,8 +51,11 @@ __device__ __forceinline__ void cmac(R& sr, R& si, R ar, R ai, R br, R bi)
     }
 }
 
-// sum over the unary coordinates of one operand at base offset `off`
-template <typename R, bool CPLX>
+// sum over the unary coordinates of one operand at base offset `off`, added in
+// order, U loads in flight. k_reduce keeps one: with four it took 3 to 47%
+// longer, with unary modes or without (a product of 20000 terms and 1000
+// outputs, complex binary64, 227 -> 332 us), for registers it does not have.
+template <typename R, bool CPLX, int U>
 __device__ __forceinline__ void unary_sum(const void* base, int64_t off, int t, int conj, int rmode, int n,
                                           int64_t size, const int64_t* ext, const int64_t* str, R& re, R& im)
 {
@@ -83,17 +86,18 @@ __device__ __forceinline__ void unary_sum(const void* base, int64_t off, int t, 
             im = round_in<R>(im, rmode);
         }
     };
-    // 4 loads in flight, added in order
     int64_t u = 0;
-    for (; u + 4 <= size; u += 4) {
-        R xr[4], xi[4];
+    if constexpr (U > 1) {
+        for (; u + U <= size; u += U) {
+            R xr[U], xi[U];
 #pragma unroll
-        for (int v = 0; v < 4; v++) {
-            load_elem<R>(base, o, t, xr[v], xi[v]);
-            next();
+            for (int v = 0; v < U; v++) {
+                load_elem<R>(base, o, t, xr[v], xi[v]);
+                next();
+            }
+#pragma unroll
+            for (int v = 0; v < U; v++) add(xr[v], xi[v]);
         }
-#pragma unroll
-        for (int v = 0; v < 4; v++) add(xr[v], xi[v]);
     }
     for (; u < size; u++) {
         R xr, xi;
@@ -174,6 +178,12 @@ __device__ __forceinline__ void free_offsets(const GenParams& p, int64_t i, int6
     }
 }
 
+// unary loads in flight in the grouped launch and the request loop: their
+// products with unary modes take 8 to 14% less time than with one (16-bit
+// storage 3% more); four spill for binary32 complex in the grouped launch
+template <typename R, bool CPLX>
+constexpr int UNARY_LOADS = CPLX && sizeof(R) == 4 ? 2 : 4;
+
 // one element of D: the reference's loop nest for output index i
 template <typename R, bool CPLX>
 __device__ __forceinline__ void element(const GenParams& p, const void* A, const void* B, const void* C, void* D,
@@ -215,8 +225,8 @@ __device__ __forceinline__ void element(const GenParams& p, const void* A, const
     }
     for (int64_t k = k0; k < p.sizeK; k++) {
         R ar, ai, br, bi;
-        unary_sum<R, CPLX>(A, kA, p.tA, p.conjA, p.round_in, p.nUA, p.sizeUA, p.UA_ext, p.UA_s, ar, ai);
-        unary_sum<R, CPLX>(B, kB, p.tB, p.conjB, p.round_in, p.nUB, p.sizeUB, p.UB_ext, p.UB_s, br, bi);
+        unary_sum<R, CPLX, UNARY_LOADS<R, CPLX>>(A, kA, p.tA, p.conjA, p.round_in, p.nUA, p.sizeUA, p.UA_ext, p.UA_s, ar, ai);
+        unary_sum<R, CPLX, UNARY_LOADS<R, CPLX>>(B, kB, p.tB, p.conjB, p.round_in, p.nUB, p.sizeUB, p.UB_ext, p.UB_s, br, bi);
         cmac<R, CPLX>(sr, si, ar, ai, br, bi);
         for (int j = 0; j < p.nK; j++) {
             kA += p.K_sA[j];
@@ -312,8 +322,8 @@ __device__ __forceinline__ void warp_element(const GenParams& p, const void* A, 
             int64_t kA, kB;
             term_offsets(k, kA, kB);
             R ar, ai, br, bi;
-            unary_sum<R, CPLX>(A, kA, p.tA, p.conjA, p.round_in, p.nUA, p.sizeUA, p.UA_ext, p.UA_s, ar, ai);
-            unary_sum<R, CPLX>(B, kB, p.tB, p.conjB, p.round_in, p.nUB, p.sizeUB, p.UB_ext, p.UB_s, br, bi);
+            unary_sum<R, CPLX, UNARY_LOADS<R, CPLX>>(A, kA, p.tA, p.conjA, p.round_in, p.nUA, p.sizeUA, p.UA_ext, p.UA_s, ar, ai);
+            unary_sum<R, CPLX, UNARY_LOADS<R, CPLX>>(B, kB, p.tB, p.conjB, p.round_in, p.nUB, p.sizeUB, p.UB_ext, p.UB_s, br, bi);
             cmac<R, CPLX>(sr, si, ar, ai, br, bi);
         }
 #pragma unroll
@@ -446,7 +456,7 @@ __device__ __forceinline__ void summed_term(const GenParams& p, const void* A, c
         xr = yr[0];
         xi = yi[0];
     } else {
-        unary_sum<R, CPLX>(B, kS, p.tB, p.conjB, p.round_in, p.nUB, p.sizeUB, p.UB_ext, p.UB_s, xr, xi);
+        unary_sum<R, CPLX, 4>(B, kS, p.tB, p.conjB, p.round_in, p.nUB, p.sizeUB, p.UB_ext, p.UB_s, xr, xi);
     }
     if (p.nUA == 0) {
 #pragma unroll
@@ -460,7 +470,7 @@ __device__ __forceinline__ void summed_term(const GenParams& p, const void* A, c
 #pragma unroll 1
         for (int r = 0; r < NR; r++) {
             R yr, yi;
-            unary_sum<R, CPLX>(A, kV + at[r], p.tA, p.conjA, p.round_in, p.nUA, p.sizeUA, p.UA_ext, p.UA_s, yr, yi);
+            unary_sum<R, CPLX, 4>(A, kV + at[r], p.tA, p.conjA, p.round_in, p.nUA, p.sizeUA, p.UA_ext, p.UA_s, yr, yi);
 #pragma unroll
             for (int q = 0; q < NR; q++)
                 if (q == r) {
@@ -731,8 +741,8 @@ __global__ void __launch_bounds__(256) k_reduce(GenParams p, const void* A, cons
                 kB += c * p.K_sB[j];
             }
             R ar, ai, br, bi;
-            unary_sum<R, CPLX>(A, kA, p.tA, p.conjA, p.round_in, p.nUA, p.sizeUA, p.UA_ext, p.UA_s, ar, ai);
-            unary_sum<R, CPLX>(B, kB, p.tB, p.conjB, p.round_in, p.nUB, p.sizeUB, p.UB_ext, p.UB_s, br, bi);
+            unary_sum<R, CPLX, 1>(A, kA, p.tA, p.conjA, p.round_in, p.nUA, p.sizeUA, p.UA_ext, p.UA_s, ar, ai);
+            unary_sum<R, CPLX, 1>(B, kB, p.tB, p.conjB, p.round_in, p.nUB, p.sizeUB, p.UB_ext, p.UB_s, br, bi);
             cmac<R, CPLX>(sr, si, ar, ai, br, bi);
         }
         sr = warp_sum(sr);
@@ -1267,7 +1277,9 @@ __device__ __forceinline__ void loop_product(const GenParams& p, const tb_ptrs& 
         element<R, CPLX>(p, q.A, q.B, q.C, q.D, i);
 }
 
-__global__ void __launch_bounds__(256) k_request_loop(LoopParams lp)
+// three blocks an SM: 80 registers. Left to itself the compiler held the four
+// products' code in 64 and spilled 452 bytes.
+__global__ void __launch_bounds__(256, 3) k_request_loop(LoopParams lp)
 {
     __shared__ GenParams sp;
     __shared__ tb_ptrs sq;
