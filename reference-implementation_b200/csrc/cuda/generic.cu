@@ -7,13 +7,17 @@
 //                  (reference_implementation/src/product.c:338-399) with the
 //                  outer loop spread over threads.
 //   k_warp_rows    the same with a warp, its lanes along the contraction
+//   k_elementwise, k_warpdot
+//                  one element of D per thread, per warp: operands of types
+//                  that are converted one by one as they are loaded
 //   k_reduce       one block per element of D for few outputs with a long
 //                  contraction: the contracted range is split over the
 //                  block's threads and combined with warp shuffles.
 //
-// Both evaluate D = op_D(alpha * sum op_A(A) op_B(B) + beta * op_C(C)) in the
+// All evaluate D = op_D(alpha * sum op_A(A) op_B(B) + beta * op_C(C)) in the
 // plan's compute domain (real/complex, binary32/binary64) and honour the
 // plan's operand rounding for the 16-bit precisions.
+#include <algorithm>
 #include <cstdio>
 #include <type_traits>
 #include <utility>
@@ -184,8 +188,9 @@ __device__ __forceinline__ void free_offsets(const GenParams& p, int64_t i, int6
 template <typename R, bool CPLX>
 constexpr int UNARY_LOADS = CPLX && sizeof(R) == 4 ? 2 : 4;
 
-// one element of D: the reference's loop nest for output index i
-template <typename R, bool CPLX>
+// one element of D: the reference's loop nest for output index i, U unary
+// loads in flight
+template <typename R, bool CPLX, int U>
 __device__ __forceinline__ void element(const GenParams& p, const void* A, const void* B, const void* C, void* D,
                                         int64_t i)
 {
@@ -225,8 +230,8 @@ __device__ __forceinline__ void element(const GenParams& p, const void* A, const
     }
     for (int64_t k = k0; k < p.sizeK; k++) {
         R ar, ai, br, bi;
-        unary_sum<R, CPLX, UNARY_LOADS<R, CPLX>>(A, kA, p.tA, p.conjA, p.round_in, p.nUA, p.sizeUA, p.UA_ext, p.UA_s, ar, ai);
-        unary_sum<R, CPLX, UNARY_LOADS<R, CPLX>>(B, kB, p.tB, p.conjB, p.round_in, p.nUB, p.sizeUB, p.UB_ext, p.UB_s, br, bi);
+        unary_sum<R, CPLX, U>(A, kA, p.tA, p.conjA, p.round_in, p.nUA, p.sizeUA, p.UA_ext, p.UA_s, ar, ai);
+        unary_sum<R, CPLX, U>(B, kB, p.tB, p.conjB, p.round_in, p.nUB, p.sizeUB, p.UB_ext, p.UB_s, br, bi);
         cmac<R, CPLX>(sr, si, ar, ai, br, bi);
         for (int j = 0; j < p.nK; j++) {
             kA += p.K_sA[j];
@@ -278,7 +283,7 @@ __device__ __forceinline__ int rows_of(const RowGroup& g, int64_t i)
 // load of the warp reads 32 neighbouring elements instead of 32 elements a
 // whole row apart, and a shuffle tree adds the 32 partial sums (a fixed
 // order: the same bits in every run).
-template <typename R, bool CPLX>
+template <typename R, bool CPLX, int U>
 __device__ __forceinline__ void warp_element(const GenParams& p, const void* A, const void* B, const void* C, void* D,
                                              int64_t i, int lane)
 {
@@ -322,8 +327,8 @@ __device__ __forceinline__ void warp_element(const GenParams& p, const void* A, 
             int64_t kA, kB;
             term_offsets(k, kA, kB);
             R ar, ai, br, bi;
-            unary_sum<R, CPLX, UNARY_LOADS<R, CPLX>>(A, kA, p.tA, p.conjA, p.round_in, p.nUA, p.sizeUA, p.UA_ext, p.UA_s, ar, ai);
-            unary_sum<R, CPLX, UNARY_LOADS<R, CPLX>>(B, kB, p.tB, p.conjB, p.round_in, p.nUB, p.sizeUB, p.UB_ext, p.UB_s, br, bi);
+            unary_sum<R, CPLX, U>(A, kA, p.tA, p.conjA, p.round_in, p.nUA, p.sizeUA, p.UA_ext, p.UA_s, ar, ai);
+            unary_sum<R, CPLX, U>(B, kB, p.tB, p.conjB, p.round_in, p.nUB, p.sizeUB, p.UB_ext, p.UB_s, br, bi);
             cmac<R, CPLX>(sr, si, ar, ai, br, bi);
         }
 #pragma unroll
@@ -335,24 +340,47 @@ __device__ __forceinline__ void warp_element(const GenParams& p, const void* A, 
     }
 }
 
-// DIRECT: both operands stored as R (pairs of R, aligned to the pair, for
-// complex), no rounding
-template <typename R, bool CPLX, bool DIRECT>
-__device__ __forceinline__ void load_term(const void* base, int64_t off, int t, int rmode, R& re, R& im)
+// How the row kernels load A and B: NATIVE, both stored as R (pairs of R,
+// aligned to the pair, for complex); STORED16, both in 16 bits, either kind
+// (R = float). Nothing branches between a step's loads, so that they are in
+// flight together; the precision's rounding is done on all of them afterwards.
+// Operands of other types (ANY) keep the kernels that take one output at a
+// time (k_elementwise, k_warpdot): in groups their loads, each behind a switch,
+// waited for one another (16-bit operands, 531 terms x 4725 outputs: 17 -> 29 us).
+enum { NATIVE, STORED16, ANY };
+
+template <typename R, bool CPLX, int LOADS>
+__device__ __forceinline__ void load_term(const void* base, int64_t off, int t, R& re, R& im)
 {
-    if constexpr (DIRECT && CPLX && sizeof(R) == 4) {
+    im = 0;
+    if constexpr (LOADS == STORED16) {
+        const unsigned short h = __ldg((const unsigned short*)base + off);
+        re = t == T_BF16 ? (R)__uint_as_float((uint32_t)h << 16) : (R)__half2float(__ushort_as_half(h));
+    } else if constexpr (CPLX && sizeof(R) == 4) {
         const float2 q = __ldg((const float2*)base + off);
         re = q.x;
         im = q.y;
-    } else if constexpr (DIRECT && CPLX) {
+    } else if constexpr (CPLX) {
         const double2 q = __ldg((const double2*)base + off);
         re = q.x;
         im = q.y;
-    } else if constexpr (DIRECT) {
-        re = __ldg((const R*)base + off);
-        im = 0;
     } else {
-        load_rounded<R>(base, off, t, rmode, re, im);
+        re = __ldg((const R*)base + off);
+    }
+}
+
+// loaded values rounded to the precision's operand format (binary32 only: the
+// 16-bit precisions compute in it)
+template <typename R, bool CPLX, int N>
+__device__ __forceinline__ void round_terms(int rmode, R (&re)[N], R (&im)[N])
+{
+    if constexpr (sizeof(R) == 4) {
+        if (rmode == TB_ROUND_NONE) return;
+#pragma unroll
+        for (int r = 0; r < N; r++) {
+            re[r] = round_in<R>(re[r], rmode);
+            if (CPLX) im[r] = round_in<R>(im[r], rmode);
+        }
     }
 }
 
@@ -407,7 +435,7 @@ __device__ __forceinline__ void fill_tables(const GenParams& p, int64_t* ka, int
 
 // unary_sum for NR rows side by side (offsets at[r] apart), from a table of
 // offsets: U coordinates' loads in flight, added in order
-template <typename R, bool CPLX, bool DIRECT, int NR, int U>
+template <typename R, bool CPLX, int LOADS, int NR, int U>
 __device__ __forceinline__ void unary_rows(const void* base, int64_t off, const int64_t (&at)[NR], int t, int conj, int rmode,
                                            const int64_t* tab, int size, R (&re)[NR], R (&im)[NR])
 {
@@ -420,7 +448,7 @@ __device__ __forceinline__ void unary_rows(const void* base, int64_t off, const 
         for (int u = 0; u < N; u++) {
             const int64_t o = off + tab[u0 + u];
 #pragma unroll
-            for (int r = 0; r < NR; r++) load_term<R, CPLX, DIRECT>(base, o + at[r], t, TB_ROUND_NONE, yr[u][r], yi[u][r]);
+            for (int r = 0; r < NR; r++) load_term<R, CPLX, LOADS>(base, o + at[r], t, yr[u][r], yi[u][r]);
         }
 #pragma unroll
         for (int u = 0; u < N; u++)
@@ -428,7 +456,7 @@ __device__ __forceinline__ void unary_rows(const void* base, int64_t off, const 
             for (int r = 0; r < NR; r++) {
                 re[r] += yr[u][r];
                 im[r] += conj ? -yi[u][r] : yi[u][r];
-                if (!DIRECT && rmode != TB_ROUND_NONE) {  // the 16-bit precisions keep the running sum in 16 bits
+                if (rmode != TB_ROUND_NONE) {  // the 16-bit precisions keep the running sum in 16 bits
                     re[r] = round_in<R>(re[r], rmode);
                     im[r] = round_in<R>(im[r], rmode);
                 }
@@ -441,18 +469,21 @@ __device__ __forceinline__ void unary_rows(const void* base, int64_t off, const 
 
 // One term's values: B's (shared) and the NR rows' of A (varying),
 // unary sums included, at contracted offsets kS and kV
-template <typename R, bool CPLX, bool DIRECT, int NR>
+template <typename R, bool CPLX, int LOADS, int NR>
 __device__ __forceinline__ void summed_term(const GenParams& p, const void* A, const void* B, int64_t kV, int64_t kS,
                                             const int64_t (&at)[NR], const int64_t* ua, const int64_t* ub, R (&vr)[NR],
                                             R (&vi)[NR], R& xr, R& xi)
 {
     if (p.nUB == 0) {
-        load_term<R, CPLX, DIRECT>(B, kS, p.tB, p.round_in, xr, xi);
-        if (p.conjB) xi = -xi;
+        R yr[1], yi[1];
+        load_term<R, CPLX, LOADS>(B, kS, p.tB, yr[0], yi[0]);
+        round_terms<R, CPLX>(p.round_in, yr, yi);
+        xr = yr[0];
+        xi = p.conjB ? -yi[0] : yi[0];
     } else if (u_tabled(p)) {
         const int64_t zero[1] = {0};
         R yr[1], yi[1];
-        unary_rows<R, CPLX, DIRECT, 1, 4>(B, kS, zero, p.tB, p.conjB, p.round_in, ub, (int)p.sizeUB, yr, yi);
+        unary_rows<R, CPLX, LOADS, 1, 4>(B, kS, zero, p.tB, p.conjB, p.round_in, ub, (int)p.sizeUB, yr, yi);
         xr = yr[0];
         xi = yi[0];
     } else {
@@ -460,12 +491,13 @@ __device__ __forceinline__ void summed_term(const GenParams& p, const void* A, c
     }
     if (p.nUA == 0) {
 #pragma unroll
-        for (int r = 0; r < NR; r++) {
-            load_term<R, CPLX, DIRECT>(A, kV + at[r], p.tA, p.round_in, vr[r], vi[r]);
+        for (int r = 0; r < NR; r++) load_term<R, CPLX, LOADS>(A, kV + at[r], p.tA, vr[r], vi[r]);
+        round_terms<R, CPLX>(p.round_in, vr, vi);
+#pragma unroll
+        for (int r = 0; r < NR; r++)
             if (p.conjA) vi[r] = -vi[r];
-        }
     } else if (u_tabled(p)) {
-        unary_rows<R, CPLX, DIRECT, NR, NR == 1 ? 4 : NR == 4 || !CPLX ? 2 : 1>(A, kV, at, p.tA, p.conjA, p.round_in, ua, (int)p.sizeUA, vr, vi);
+        unary_rows<R, CPLX, LOADS, NR, NR == 1 ? 4 : NR == 4 || !CPLX ? 2 : 1>(A, kV, at, p.tA, p.conjA, p.round_in, ua, (int)p.sizeUA, vr, vi);
     } else {
 #pragma unroll 1
         for (int r = 0; r < NR; r++) {
@@ -482,7 +514,7 @@ __device__ __forceinline__ void summed_term(const GenParams& p, const void* A, c
 }
 
 // NR outputs per thread: element() for each of them (NR = 1: the plain element kernel)
-template <typename R, bool CPLX, bool DIRECT, int NR>
+template <typename R, bool CPLX, int LOADS, int NR>
 __global__ void __launch_bounds__(256) k_element_rows(GenParams p, RowGroup g,
                                                       const void* A, const void* B, const void* C, void* D)
 {
@@ -533,9 +565,14 @@ __global__ void __launch_bounds__(256) k_element_rows(GenParams p, RowGroup g,
             for (int u = 0; u < U; u++) {
                 int64_t v, s;
                 offsets(k + u, v, s);
-                load_term<R, CPLX, DIRECT>(B, s, p.tB, p.round_in, xr[u], xi[u]);
+                load_term<R, CPLX, LOADS>(B, s, p.tB, xr[u], xi[u]);
 #pragma unroll
-                for (int r = 0; r < NR; r++) load_term<R, CPLX, DIRECT>(A, v + at[r], p.tA, p.round_in, vr[u][r], vi[u][r]);
+                for (int r = 0; r < NR; r++) load_term<R, CPLX, LOADS>(A, v + at[r], p.tA, vr[u][r], vi[u][r]);
+            }
+            if (sizeof(R) == 4 && p.round_in != TB_ROUND_NONE) {
+                round_terms<R, CPLX>(p.round_in, xr, xi);
+#pragma unroll
+                for (int u = 0; u < U; u++) round_terms<R, CPLX>(p.round_in, vr[u], vi[u]);
             }
 #pragma unroll
             for (int u = 0; u < U; u++) {
@@ -553,7 +590,7 @@ __global__ void __launch_bounds__(256) k_element_rows(GenParams p, RowGroup g,
                 int64_t v, s;
                 offsets(k, v, s);
                 R vr[NR], vi[NR], xr, xi;
-                summed_term<R, CPLX, DIRECT, NR>(p, A, B, v, s, at, ua, ub, vr, vi, xr, xi);
+                summed_term<R, CPLX, LOADS, NR>(p, A, B, v, s, at, ua, ub, vr, vi, xr, xi);
 #pragma unroll
                 for (int r = 0; r < NR; r++) add(r, vr[r], vi[r], xr, xi);
             }
@@ -575,7 +612,7 @@ __global__ void __launch_bounds__(256) k_element_rows(GenParams p, RowGroup g,
 // in which a lane hands away half of its rows at each step, so 8 rows take 9
 // shuffles instead of 40 and end on 8 different lanes; each row's sum is that
 // of the same tree as warp_element's. UNARY: some operand has unary modes.
-template <typename R, bool CPLX, bool DIRECT, int NR, bool UNARY>
+template <typename R, bool CPLX, int LOADS, int NR, bool UNARY>
 __global__ void __launch_bounds__(128, CPLX && NR == 8 ? (sizeof(R) == 4 ? 4 : 2) : sizeof(R) == 8 ? 4 : CPLX || UNARY ? 5 : 8)
     k_warp_rows(GenParams p, RowGroup g, const void* A, const void* B,
                 const void* C, void* D)
@@ -624,9 +661,18 @@ __global__ void __launch_bounds__(128, CPLX && NR == 8 ? (sizeof(R) == 4 ? 4 : 2
                     if (k + 32 * u >= p.sizeK) continue;
                     int64_t v, s;
                     offsets(k + 32 * u, v, s);
-                    load_term<R, CPLX, DIRECT>(B, s, p.tB, p.round_in, xr[u], xi[u]);
+                    load_term<R, CPLX, LOADS>(B, s, p.tB, xr[u], xi[u]);
 #pragma unroll
-                    for (int r = 0; r < NR; r++) load_term<R, CPLX, DIRECT>(A, v + at[r], p.tA, p.round_in, vr[u][r], vi[u][r]);
+                    for (int r = 0; r < NR; r++) load_term<R, CPLX, LOADS>(A, v + at[r], p.tA, vr[u][r], vi[u][r]);
+                }
+                if (sizeof(R) == 4 && p.round_in != TB_ROUND_NONE) {
+#pragma unroll
+                    for (int u = 0; u < UNR; u++) {
+                        if (k + 32 * u >= p.sizeK) continue;
+                        xr[u] = round_in<R>(xr[u], p.round_in);
+                        if (CPLX) xi[u] = round_in<R>(xi[u], p.round_in);
+                        round_terms<R, CPLX>(p.round_in, vr[u], vi[u]);
+                    }
                 }
 #pragma unroll
                 for (int u = 0; u < UNR; u++) {
@@ -641,7 +687,7 @@ __global__ void __launch_bounds__(128, CPLX && NR == 8 ? (sizeof(R) == 4 ? 4 : 2
                 int64_t v, s;
                 offsets(k, v, s);
                 R vr[NR], vi[NR], xr, xi;
-                summed_term<R, CPLX, DIRECT, NR>(p, A, B, v, s, at, ua, ub, vr, vi, xr, xi);
+                summed_term<R, CPLX, LOADS, NR>(p, A, B, v, s, at, ua, ub, vr, vi, xr, xi);
 #pragma unroll
                 for (int r = 0; r < NR; r++) add(r, vr[r], vi[r], xr, xi);
             }
@@ -670,6 +716,22 @@ __global__ void __launch_bounds__(128, CPLX && NR == 8 ? (sizeof(R) == 4 ? 4 : 2
     }
 }
 
+template <typename R, bool CPLX>
+__global__ void __launch_bounds__(256) k_elementwise(GenParams p, const void* A, const void* B, const void* C, void* D)
+{
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < p.sizeF; i += stride)
+        element<R, CPLX, 1>(p, A, B, C, D, i);
+}
+
+template <typename R, bool CPLX>
+__global__ void __launch_bounds__(256) k_warpdot(GenParams p, const void* A, const void* B, const void* C, void* D)
+{
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+    for (int64_t i = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < p.sizeF; i += warps)
+        warp_element<R, CPLX, 1>(p, A, B, C, D, i, threadIdx.x & 31);
+}
+
 // Many independent products of the same compute domain in one launch:
 // product j owns blocks [first[j], first[j+1]) and walks its elements with
 // them. Descriptors and operand pointers live in device memory.
@@ -691,12 +753,12 @@ __global__ void __launch_bounds__(256) k_elementwise_group(const GenParams* __re
         const int64_t warps = nb * (blockDim.x >> 5);
         for (int64_t i = ((int64_t)blockIdx.x - first[lo]) * (blockDim.x >> 5) + (threadIdx.x >> 5); i < p.sizeF;
              i += warps)
-            warp_element<R, CPLX>(p, q.A, q.B, q.C, q.D, i, threadIdx.x & 31);
+            warp_element<R, CPLX, UNARY_LOADS<R, CPLX>>(p, q.A, q.B, q.C, q.D, i, threadIdx.x & 31);
         return;
     }
     const int64_t stride = nb * blockDim.x;
     for (int64_t i = ((int64_t)blockIdx.x - first[lo]) * blockDim.x + threadIdx.x; i < p.sizeF; i += stride)
-        element<R, CPLX>(p, q.A, q.B, q.C, q.D, i);
+        element<R, CPLX, UNARY_LOADS<R, CPLX>>(p, q.A, q.B, q.C, q.D, i);
 }
 
 template <typename R>
@@ -832,7 +894,7 @@ static void fill_params(const tb_plan* P, GenParams& g)
     g.warp = warpdot_ok(g) ? 1 : 0;
 }
 
-// Element path kernel: the warp per output (k_warp_rows)
+// Element path kernel: the warp per output (k_warp_rows, k_warpdot)
 //   - when an operand is contiguous along the contraction while consecutive
 //     outputs step it by a stride other than 0 or 1 (one thread per output
 //     would read it a row apart from lane to lane), for contractions of at
@@ -968,7 +1030,22 @@ static int warp_rows(GenParams& g, RowGroup& q)
     return 1;
 }
 
-template <typename R, bool CPLX, bool DIRECT>
+// How the row kernels would load the operands of a product computed in the
+// type of storage `stored`.
+static int loads_of(const GenParams& g, int stored)
+{
+    if (g.tA == stored && g.tB == stored) return NATIVE;
+    return stored == T_F32 && g.tA >= T_F16 && g.tB >= T_F16 ? STORED16 : ANY;
+}
+
+// Rows per step of the row kernels, g then in groups, or 0: one output at a time.
+static int rows_of_step(GenParams& g, RowGroup& q, int loads)
+{
+    if (loads == ANY) return 0;
+    return g.warp ? warp_rows(g, q) : thread_rows(g, q);
+}
+
+template <typename R, bool CPLX, int LOADS>
 static void launch_rows(const GenParams& g, const RowGroup& q, int nr, const tb_ptrs* d, cudaStream_t s)
 {
     const int per = g.warp ? 4 : 256, threads = g.warp ? 128 : 256;  // groups and threads of a block
@@ -977,14 +1054,14 @@ static void launch_rows(const GenParams& g, const RowGroup& q, int nr, const tb_
     if (blocks < 1) blocks = 1;
     void (*kern)(GenParams, RowGroup, const void*, const void*, const void*, void*);
     if (g.warp && (g.nUA || g.nUB))
-        kern = nr == 8 ? k_warp_rows<R, CPLX, DIRECT, 8, true>
-               : nr == 4 ? k_warp_rows<R, CPLX, DIRECT, 4, true> : k_warp_rows<R, CPLX, DIRECT, 1, true>;
+        kern = nr == 8 ? k_warp_rows<R, CPLX, LOADS, 8, true>
+               : nr == 4 ? k_warp_rows<R, CPLX, LOADS, 4, true> : k_warp_rows<R, CPLX, LOADS, 1, true>;
     else if (g.warp)
-        kern = nr == 8 ? k_warp_rows<R, CPLX, DIRECT, 8, false>
-               : nr == 4 ? k_warp_rows<R, CPLX, DIRECT, 4, false> : k_warp_rows<R, CPLX, DIRECT, 1, false>;
+        kern = nr == 8 ? k_warp_rows<R, CPLX, LOADS, 8, false>
+               : nr == 4 ? k_warp_rows<R, CPLX, LOADS, 4, false> : k_warp_rows<R, CPLX, LOADS, 1, false>;
     else
-        kern = nr == 8 ? k_element_rows<R, CPLX, DIRECT, 8>
-               : nr == 4 ? k_element_rows<R, CPLX, DIRECT, 4> : k_element_rows<R, CPLX, DIRECT, 1>;
+        kern = nr == 8 ? k_element_rows<R, CPLX, LOADS, 8>
+               : nr == 4 ? k_element_rows<R, CPLX, LOADS, 4> : k_element_rows<R, CPLX, LOADS, 1>;
     kern<<<(unsigned)blocks, threads, 0, s>>>(g, q, q.swapped ? d->B : d->A, q.swapped ? d->A : d->B, d->C, d->D);
 }
 
@@ -1019,14 +1096,21 @@ static cudaError_t launch_typed(GenParams& g, int path, const tb_ptrs* d, cudaSt
         cudaFreeAsync(ws, s);
         return e;
     }
+    const uintptr_t pair = CPLX ? 2 * sizeof(R) : 1;  // complex pairs are loaded whole
+    const bool aligned = (uintptr_t)d->A % pair == 0 && (uintptr_t)d->B % pair == 0;
+    const int loads = aligned ? loads_of(g, stored) : ANY;
     RowGroup q;
     memset(&q, 0, sizeof(q));
-    const int nr = g.warp ? warp_rows(g, q) : thread_rows(g, q);
-    const uintptr_t pair = CPLX ? 2 * sizeof(R) : 1;  // complex pairs are loaded whole
-    if (g.tA == stored && g.tB == stored && g.round_in == TB_ROUND_NONE && (uintptr_t)d->A % pair == 0 && (uintptr_t)d->B % pair == 0)
-        launch_rows<R, CPLX, true>(g, q, nr, d, s);
-    else
-        launch_rows<R, CPLX, false>(g, q, nr, d, s);
+    const int nr = rows_of_step(g, q, loads);
+    if (nr == 0) {
+        const int per = g.warp ? 8 : 256;  // outputs of a block
+        const int64_t most = 148 * (g.warp ? 32 : 64), blocks = std::max<int64_t>(1, std::min((g.sizeF + per - 1) / per, most));
+        (g.warp ? k_warpdot<R, CPLX> : k_elementwise<R, CPLX>)<<<(unsigned)blocks, 256, 0, s>>>(g, d->A, d->B, d->C, d->D);
+    } else if (loads == NATIVE) {
+        launch_rows<R, CPLX, NATIVE>(g, q, nr, d, s);
+    } else if constexpr (sizeof(R) == 4 && !CPLX) {
+        launch_rows<R, CPLX, STORED16>(g, q, nr, d, s);
+    }
     count_launch();
     return cudaGetLastError();
 }
@@ -1269,12 +1353,12 @@ __device__ __forceinline__ void loop_product(const GenParams& p, const tb_ptrs& 
     if (warp) {
         const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
         for (int64_t i = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < p.sizeF; i += warps)
-            warp_element<R, CPLX>(p, q.A, q.B, q.C, q.D, i, threadIdx.x & 31);
+            warp_element<R, CPLX, UNARY_LOADS<R, CPLX>>(p, q.A, q.B, q.C, q.D, i, threadIdx.x & 31);
         return;
     }
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < p.sizeF; i += stride)
-        element<R, CPLX>(p, q.A, q.B, q.C, q.D, i);
+        element<R, CPLX, UNARY_LOADS<R, CPLX>>(p, q.A, q.B, q.C, q.D, i);
 }
 
 // three blocks an SM: 80 registers. Left to itself the compiler held the four
@@ -1401,11 +1485,18 @@ cudaError_t loop_launch(void* slots_dev, void* state, int nslots, int blocks, un
 
 }  // namespace tb
 
-// Kernel of the element path for a plan: 0 one thread per output, 1 one warp
-// per output (k_warp_rows). No device call.
-extern "C" int tbk_generic_kernel(const tb_plan* P)
+// Kernel of the element path for a plan: 0 threads, 1 warps. *rows: outputs of
+// a step along a mode (0: no row kernel), *spread and *swapped: RowGroup's, for
+// operands aligned to their elements. No device call.
+extern "C" int tbk_generic_kernel(const tb_plan* P, int* rows, int* spread, int* swapped)
 {
+    static const int stored[4] = {T_F32, T_F64, T_C32, T_C64};  // by TB_R32 .. TB_C64
     tb::GenParams g;
     tb::fill_params(P, g);
+    tb::RowGroup q;
+    memset(&q, 0, sizeof(q));
+    *rows = tb::rows_of_step(g, q, tb::loads_of(g, stored[P->compute]));
+    *spread = q.spread;
+    *swapped = q.swapped;
     return g.warp;
 }

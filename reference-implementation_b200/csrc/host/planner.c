@@ -535,9 +535,12 @@ size_t tb_describe(const tb_plan* p, size_t maxlen, char* out)
         at = put(out, maxlen, at, " operands=%s", tbk_tc_split_in_place(p) ? "in_place" : "packed");
     if (p->path == TB_PATH_SLICED) at = put(out, maxlen, at, " slices=%d", p->slices);
     if (p->path == TB_PATH_GENERIC) {
-        const int warp = tbk_generic_kernel(p);
+        int rows, spread, swapped;
+        const int warp = tbk_generic_kernel(p, &rows, &spread, &swapped);
         at = put(out, maxlen, at, " kernel=%s", warp ? "warpdot" : "element");
         if (!warp && p->elem_stage) at = put(out, maxlen, at, " staged=%s", p->elem_stage == 1 ? "A" : "B");
+        at = put(out, maxlen, at, " rows=%d", rows);
+        if (rows > 1) at = put(out, maxlen, at, " spread=%d along=%s", spread, swapped ? "B" : "A");
     }
     if (p->path == TB_PATH_SIMT) {
         static const char* kern[] = {"tiled", "narrow", "narrow_stream", "narrow_coop", "narrow_cstream", "narrow_vec",

@@ -1,0 +1,54 @@
+"""Which CUDA-core kernel a product runs, as tapp_b200_describe_plan reports
+it (no GPU): the rules of the element path and of the tiled GEMM, at sizes on
+both sides of their lines.
+"""
+import re
+
+import pytest
+
+import tapp_b200
+from tapp_b200.abi import TAPP_F32, TAPP_F64, TAPP_C32, TAPP_C64, TAPP_F16, TAPP_BF16
+
+
+def plan_text(tapp, a, b, d, ext, types, prec, path=0):
+    """The plan of D[d] = sum A[a] B[b] + C[d], one letter per mode, dense column-major; types of A, B, C, D"""
+    infos = []
+    for labels, t in zip((a, b, d, d), types):
+        strides, at = [], 1
+        for x in labels:
+            strides.append(at)
+            at *= ext[x]
+        infos.append(tapp.tensor_info(t, [ext[x] for x in labels], strides)[1])
+    err, plan = tapp.create_product(0, [0] * 4, infos, [[ord(x) for x in labels] for labels in (a, b, d, d)], prec)
+    assert err == 0
+    ex = tapp.create_executor()
+    if path:
+        tapp.set_int(ex, tapp_b200.ATTR_PATH, path)
+    text = tapp.describe(plan, ex)
+    tapp.lib.TAPP_destroy_executor(ex)
+    tapp.lib.TAPP_destroy_tensor_product(plan)
+    for h in infos:
+        tapp.lib.TAPP_destroy_tensor_info(h)
+    return text
+
+
+def field(text, name):
+    m = re.search(rf" {name}=(\S+)", text)
+    return m and m[1]
+
+
+# operands stored as computed, rounded or not, and 16-bit operands of either kind are loaded in groups; what is converted
+# behind a switch is taken one output at a time, threads and warps alike
+@pytest.mark.parametrize("types,prec,grouped", [
+    ((TAPP_F32,) * 4, 0, True), ((TAPP_F32,) * 4, 6, True), ((TAPP_F16,) * 4, 5, True), ((TAPP_F16,) * 4, -1, True),
+    ((TAPP_BF16, TAPP_F16, TAPP_F32, TAPP_F32), -1, True), ((TAPP_F64,) * 4, -1, True), ((TAPP_C32,) * 4, 6, True),
+    ((TAPP_C64,) * 4, -1, True), ((TAPP_F32, TAPP_BF16, TAPP_F32, TAPP_F32), -1, False),
+    ((TAPP_F64, TAPP_F64, TAPP_F32, TAPP_F32), 0, False), ((TAPP_F32, TAPP_F32, TAPP_F32, TAPP_F32), 1, False),
+    ((TAPP_F16, TAPP_F16, TAPP_C32, TAPP_C32), -1, False), ((TAPP_C64, TAPP_C32, TAPP_C64, TAPP_C64), -1, False)])
+def test_element_operands_loaded_in_groups(tapp, types, prec, grouped):
+    ext = {"a": 500, "b": 401, "d": 9, "k": 5}
+    t = plan_text(tapp, "abkd", "bka", "dab", ext, types, prec)
+    assert field(t, "kernel") == "element" and field(t, "rows") == ("8" if grouped else "0"), t
+    ext = {"a": 40, "b": 51, "d": 9, "k": 70}
+    t = plan_text(tapp, "kabd", "kab", "dab", ext, types, prec)
+    assert field(t, "kernel") == "warpdot" and field(t, "rows") == ("8" if grouped else "0"), t
