@@ -1038,11 +1038,20 @@ static int loads_of(const GenParams& g, int stored)
     return stored == T_F32 && g.tA >= T_F16 && g.tB >= T_F16 ? STORED16 : ANY;
 }
 
-// Rows per step of the row kernels, g then in groups, or 0: one output at a time.
+// Rows per step of the row kernels, g then in groups, or 0: one output at a
+// time. A single term without a mode to group by gains nothing from the offset
+// tables and pays for filling them (binary32, 889200 outputs 12.1 us without,
+// 14.6 with; 0.97 on average over 283 products, 0.81 at worst), and a rounded
+// complex one nothing from groups (3.9 million outputs 64 us one by one, 77 in
+// groups of 8).
 static int rows_of_step(GenParams& g, RowGroup& q, int loads)
 {
     if (loads == ANY) return 0;
-    return g.warp ? warp_rows(g, q) : thread_rows(g, q);
+    if (g.warp) return warp_rows(g, q);
+    const bool one_term = g.sizeK == 1 && !g.nUA && !g.nUB;
+    if (one_term && g.tA == T_C32 && g.round_in != TB_ROUND_NONE) return 0;
+    const int nr = thread_rows(g, q);
+    return nr == 1 && one_term ? 0 : nr;
 }
 
 template <typename R, bool CPLX, int LOADS>

@@ -52,3 +52,16 @@ def test_element_operands_loaded_in_groups(tapp, types, prec, grouped):
     ext = {"a": 40, "b": 51, "d": 9, "k": 70}
     t = plan_text(tapp, "kabd", "kab", "dab", ext, types, prec)
     assert field(t, "kernel") == "warpdot" and field(t, "rows") == ("8" if grouped else "0"), t
+
+
+# a single term is not worth filling offset tables for, unless outputs share loads of an operand
+@pytest.mark.parametrize("a,b,ext,types,prec,rows", [
+    ("abd", "ba", {"a": 78, "b": 25, "d": 19}, (TAPP_F32,) * 4, 0, "0"),
+    ("abd", "ba", {"a": 780, "b": 250, "d": 19}, (TAPP_F32,) * 4, 0, "8"),
+    ("abd", "ba", {"a": 780, "b": 250, "d": 19}, (TAPP_C32,) * 4, -1, "8"),
+    ("abd", "ba", {"a": 780, "b": 250, "d": 19}, (TAPP_C32,) * 4, 6, "0"),
+    ("abdk", "ba", {"a": 78, "b": 25, "d": 19, "k": 3}, (TAPP_F32,) * 4, 0, "1"),
+    ("abdk", "bak", {"a": 78, "b": 25, "d": 19, "k": 2}, (TAPP_F32,) * 4, 0, "1")])
+def test_one_term_takes_one_output_at_a_time(tapp, a, b, ext, types, prec, rows):
+    t = plan_text(tapp, a, b, "abd", ext, types, prec)
+    assert field(t, "kernel") == "element" and field(t, "rows") == rows, t
