@@ -979,14 +979,17 @@ static bool one_operand_lacks(const GenParams& g, int j) { return (g.F_sA[j] == 
 // of a warp read), and of several the one along which D is nearest; where
 // only the first one qualifies, spread over it as long as 8 neighbours are
 // left to the lanes (32 bytes of binary32). 8 or 4 rows as long as the threads
-// fill the GPU about once (148 x 1024) and the mode half a group.
+// fill the GPU about once (148 x 1024) and the mode more than half a group: the
+// rows it lacks still cost loads (modes of 4, against one output a thread: 8
+// rows 0.70 to 1.43, 4 rows 1.05 to 1.76; modes of 2: 4 rows 0.83 to 1.6, one
+// row 1.04 and more).
 static int thread_rows(GenParams& g, RowGroup& q)
 {
     if (g.nUA || g.nUB || g.sizeK < 1) return 1;
     int best = -1;
     auto a = [](int64_t x) { return x < 0 ? -x : x; };
     for (int j = 1; j < g.nF; j++)
-        if (one_operand_lacks(g, j) && 2 * g.F_ext[j] >= 4 && (best < 0 || a(g.F_sD[j]) < a(g.F_sD[best]))) best = j;
+        if (one_operand_lacks(g, j) && 2 * g.F_ext[j] > 4 && (best < 0 || a(g.F_sD[j]) < a(g.F_sD[best]))) best = j;
     const bool spread = best < 0;
     if (spread) {
         if (g.nF < 1 || !one_operand_lacks(g, 0)) return 1;
@@ -995,7 +998,7 @@ static int thread_rows(GenParams& g, RowGroup& q)
     const int64_t e = g.F_ext[best], others = g.sizeF / e;
     for (int nr = 8; nr >= 4; nr /= 2) {
         const int64_t groups = (e + nr - 1) / nr;
-        if (2 * e < nr || others * groups < 148 * 1024 || (spread && groups < 8)) continue;
+        if (2 * e <= nr || others * groups < 148 * 1024 || (spread && groups < 8)) continue;
         group_rows(g, q, best, nr, spread);
         return nr;
     }

@@ -65,3 +65,13 @@ def test_element_operands_loaded_in_groups(tapp, types, prec, grouped):
 def test_one_term_takes_one_output_at_a_time(tapp, a, b, ext, types, prec, rows):
     t = plan_text(tapp, a, b, "abd", ext, types, prec)
     assert field(t, "kernel") == "element" and field(t, "rows") == rows, t
+
+
+# groups that the mode fills no more than half are not formed
+@pytest.mark.parametrize("d,k,types,rows", [
+    (4, 3, (TAPP_F32,) * 4, "4"), (5, 3, (TAPP_F32,) * 4, "8"), (4, 3, (TAPP_F64,) * 4, "4"), (3, 3, (TAPP_F64,) * 4, "4"),
+    (2, 3, (TAPP_F64,) * 4, "1"), (2, 3, (TAPP_F32,) * 4, "1"), (2, 3, (TAPP_BF16,) * 4, "1"),
+    (2, 1, (TAPP_F32,) * 4, "0"), (3, 1, (TAPP_F32,) * 4, "4")])
+def test_rows_fill_more_than_half_a_group(tapp, d, k, types, rows):
+    t = plan_text(tapp, "abkd", "bka", "abd", {"a": 500, "b": 401, "d": d, "k": k}, types, -1)
+    assert field(t, "kernel") == "element" and field(t, "rows") == rows, t
