@@ -394,7 +394,7 @@ __device__ __forceinline__ void round_terms(int rmode, R (&re)[N], R (&im)[N])
 constexpr int TAB_K = 512, TAB_U = 128;
 
 __device__ __forceinline__ bool k_tabled(const GenParams& p) { return p.sizeK <= TAB_K; }
-__device__ __forceinline__ bool u_tabled(const GenParams& p) { return p.sizeUA <= TAB_U && p.sizeUB <= TAB_U; }
+__host__ __device__ __forceinline__ bool u_tabled(const GenParams& p) { return p.sizeUA <= TAB_U && p.sizeUB <= TAB_U; }
 
 __device__ __forceinline__ void fill_tables(const GenParams& p, int64_t* ka, int64_t* kb, int64_t* ua, int64_t* ub)
 {
@@ -468,7 +468,8 @@ __device__ __forceinline__ void unary_rows(const void* base, int64_t off, const 
 }
 
 // One term's values: B's (shared) and the NR rows' of A (varying),
-// unary sums included, at contracted offsets kS and kV
+// unary sums included, at contracted offsets kS and kV. (Several rows are only
+// taken where the tables hold the unary modes.)
 template <typename R, bool CPLX, int LOADS, int NR>
 __device__ __forceinline__ void summed_term(const GenParams& p, const void* A, const void* B, int64_t kV, int64_t kS,
                                             const int64_t (&at)[NR], const int64_t* ua, const int64_t* ub, R (&vr)[NR],
@@ -480,7 +481,7 @@ __device__ __forceinline__ void summed_term(const GenParams& p, const void* A, c
         round_terms<R, CPLX>(p.round_in, yr, yi);
         xr = yr[0];
         xi = p.conjB ? -yi[0] : yi[0];
-    } else if (u_tabled(p)) {
+    } else if (NR > 1 || u_tabled(p)) {
         const int64_t zero[1] = {0};
         R yr[1], yi[1];
         unary_rows<R, CPLX, LOADS, 1, 4>(B, kS, zero, p.tB, p.conjB, p.round_in, ub, (int)p.sizeUB, yr, yi);
@@ -496,20 +497,10 @@ __device__ __forceinline__ void summed_term(const GenParams& p, const void* A, c
 #pragma unroll
         for (int r = 0; r < NR; r++)
             if (p.conjA) vi[r] = -vi[r];
-    } else if (u_tabled(p)) {
+    } else if (NR > 1 || u_tabled(p)) {
         unary_rows<R, CPLX, LOADS, NR, NR == 1 ? 4 : NR == 4 || !CPLX ? 2 : 1>(A, kV, at, p.tA, p.conjA, p.round_in, ua, (int)p.sizeUA, vr, vi);
     } else {
-#pragma unroll 1
-        for (int r = 0; r < NR; r++) {
-            R yr, yi;
-            unary_sum<R, CPLX, 4>(A, kV + at[r], p.tA, p.conjA, p.round_in, p.nUA, p.sizeUA, p.UA_ext, p.UA_s, yr, yi);
-#pragma unroll
-            for (int q = 0; q < NR; q++)
-                if (q == r) {
-                    vr[q] = yr;
-                    vi[q] = yi;
-                }
-        }
+        unary_sum<R, CPLX, 4>(A, kV + at[0], p.tA, p.conjA, p.round_in, p.nUA, p.sizeUA, p.UA_ext, p.UA_s, vr[0], vi[0]);
     }
 }
 
@@ -972,6 +963,17 @@ static void group_rows(GenParams& g, RowGroup& q, int j, int nr, bool spread)
     g.sizeF = others * groups;
 }
 
+static int stored_bytes(int t)
+{
+    switch (t) {
+    case T_F32: return 4;
+    case T_F64: return 8;
+    case T_C32: return 8;
+    case T_C64: return 16;
+    default: return 2;
+    }
+}
+
 static bool one_operand_lacks(const GenParams& g, int j) { return (g.F_sA[j] == 0) != (g.F_sB[j] == 0); }
 
 // Rows per thread of k_element_rows, or 1: a mode that one
@@ -1010,8 +1012,18 @@ static int thread_rows(GenParams& g, RowGroup& q)
 // lacks the one with the fewest loads (a group's NR of the varying operand and
 // one of the shared, over rounds of the 16 warps per SM that run at a time),
 // of equal ones the nearest in D.
+// One row where unary modes are longer than the offset tables: a group would
+// step through them row by row, with one row's loads in flight (133 unary
+// values, 51 terms, 5664 outputs 231 us in k_warpdot, 322 in groups of 4); and
+// where a lane reads runs of 64 bytes and more along one: the 32 lanes' lines of
+// 8 rows do not stay in L1 (75 contiguous complex values, 26 terms, 18513 outputs
+// 235 us in k_warpdot, 710 in groups of 8, below 200 with one row).
 static int warp_rows(GenParams& g, RowGroup& q)
 {
+    auto long_runs = [](int n, const int64_t* ext, const int64_t* str, int t) {
+        return n > 0 && (str[0] == 1 || str[0] == -1) && ext[0] * stored_bytes(t) >= 64;
+    };
+    if (!u_tabled(g) || long_runs(g.nUA, g.UA_ext, g.UA_s, g.tA) || long_runs(g.nUB, g.UB_ext, g.UB_s, g.tB)) return 1;
     auto a = [](int64_t x) { return x < 0 ? -x : x; };
     for (int nr = 8; nr >= 4; nr /= 2) {
         int best = -1;
@@ -1046,10 +1058,13 @@ static int loads_of(const GenParams& g, int stored)
 // tables and pays for filling them (binary32, 889200 outputs 12.1 us without,
 // 14.6 with; 0.97 on average over 283 products, 0.81 at worst), and a rounded
 // complex one nothing from groups (3.9 million outputs 64 us one by one, 77 in
-// groups of 8).
+// groups of 8). Unary modes beyond the tables, rounded or of 16 bits, convert
+// one value after the other whichever kernel sums them, and the tables' shared
+// memory is missing from L1 (135 rounded complex values, 36 terms, 7350 outputs
+// 293 us in k_warpdot, 655 in k_warp_rows).
 static int rows_of_step(GenParams& g, RowGroup& q, int loads)
 {
-    if (loads == ANY) return 0;
+    if (loads == ANY || (!u_tabled(g) && (loads == STORED16 || g.round_in != TB_ROUND_NONE))) return 0;
     if (g.warp) return warp_rows(g, q);
     const bool one_term = g.sizeK == 1 && !g.nUA && !g.nUB;
     if (one_term && g.tA == T_C32 && g.round_in != TB_ROUND_NONE) return 0;
@@ -1203,17 +1218,6 @@ __global__ void __launch_bounds__(256) k_stage(StageParams p)
             for (int w = 0; w < p.words; w++)
                 ((uint32_t*)p.dst)[i * p.words + w] = __ldg((const uint32_t*)p.src + o * p.words + w);
         }
-    }
-}
-
-static int stored_bytes(int t)
-{
-    switch (t) {
-    case T_F32: return 4;
-    case T_F64: return 8;
-    case T_C32: return 8;
-    case T_C64: return 16;
-    default: return 2;
     }
 }
 

@@ -75,3 +75,15 @@ def test_one_term_takes_one_output_at_a_time(tapp, a, b, ext, types, prec, rows)
 def test_rows_fill_more_than_half_a_group(tapp, d, k, types, rows):
     t = plan_text(tapp, "abkd", "bka", "abd", {"a": 500, "b": 401, "d": d, "k": k}, types, -1)
     assert field(t, "kernel") == "element" and field(t, "rows") == rows, t
+
+
+# unary modes beyond the offset tables are summed for one output a warp, in k_warpdot where each value is converted; and so
+# are contiguous ones whose runs fill lines
+@pytest.mark.parametrize("a,types,prec,u,v,rows", [
+    ("ahku", (TAPP_F32,) * 4, 0, 128, 128, "8"), ("ahku", (TAPP_F32,) * 4, 0, 129, 3, "1"), ("ahku", (TAPP_F32,) * 4, 0, 3, 129, "1"),
+    ("ahku", (TAPP_C64,) * 4, -1, 129, 3, "1"), ("ahku", (TAPP_F32,) * 4, 6, 129, 3, "0"), ("ahku", (TAPP_F16,) * 4, -1, 129, 3, "0"),
+    ("ahku", (TAPP_F16,) * 4, -1, 128, 3, "8"), ("uahk", (TAPP_F32,) * 4, 0, 15, 3, "8"), ("uahk", (TAPP_F32,) * 4, 0, 16, 3, "1"),
+    ("uahk", (TAPP_C32,) * 4, -1, 8, 3, "1"), ("uahk", (TAPP_F16,) * 4, -1, 31, 3, "8"), ("uahk", (TAPP_F16,) * 4, -1, 32, 3, "1")])
+def test_long_unary_modes_take_one_row(tapp, a, types, prec, u, v, rows):
+    t = plan_text(tapp, a, "khv", "ah", {"a": 150, "h": 120, "k": 33, "u": u, "v": v}, types, prec)
+    assert field(t, "kernel") == "warpdot" and field(t, "rows") == rows, t
