@@ -1,4 +1,4 @@
-"""GPU parity of the element path's warp-per-output kernel (k_warpdot):
+"""GPU parity of the element path's warp-per-output kernels (k_warp_rows, k_warpdot):
 products whose contraction runs along an operand's contiguous mode while
 consecutive outputs step that operand by a whole row (batched
 matrix-vector and Hadamard products with A stored contraction-fastest).

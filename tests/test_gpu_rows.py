@@ -53,8 +53,8 @@ def check(tapp, oracle, case, kernel):
     assert run.D.buf.view(np.uint8).tobytes() == one == two
 
 
-# the mode d is A's alone: fewer rows than a group, one group and a remainder, walked last or first; the batch is large
-# enough for 8 (or only 4) rows a thread
+# the mode d is A's alone, walked last or first; the batch is large enough for 4 rows a thread at most
+# (test_gpu_row_forms.py has the others)
 @pytest.mark.parametrize("storage,prec", TYPES)
 @pytest.mark.parametrize("d,batch", [(3, 200), (8, 160), (21, 110), (5, 300)])
 @pytest.mark.parametrize("a,b,o", [("abkd", "bka", "dab"), ("abkd", "kab", "abd"), ("dabk", "abk", "dab")])
