@@ -2416,3 +2416,17 @@ extern "C" int tbk_simt_kernel(const tb_plan* P)
     const int kind = narrow_kind(P, p, nb);
     return tb::tile_over_narrow(p, P->compute, kind) ? 0 : kind;
 }
+
+// Rows and columns of k_tile's tile, blocks of a cluster and splits through
+// the workspace for a plan that runs it; 0 where another kernel does (k_simt:
+// operands converted at load). No device call.
+extern "C" int tbk_simt_tile(const tb_plan* P, int out[4])
+{
+    using namespace tb;
+    simt::Params p;
+    tb_ptrs d = {nullptr, nullptr, nullptr, nullptr};
+    simt_params(P, &d, p);
+    if (tbk_simt_kernel(P) != 0 || !tile_takes(p, P->compute)) return 0;
+    tile_describe(p, P->compute, simt_scratch_bytes(P), out);
+    return 1;
+}

@@ -65,6 +65,7 @@ __device__ __forceinline__ void epilogue_value(const P& p, T xr, T xi, T cr, T c
 bool tile_takes(const simt::Params& p, int compute);
 // ... and whether it takes a product that the narrow kernels could run
 bool tile_over_narrow(const simt::Params& p, int compute, int kind);
+void tile_describe(const simt::Params& p, int compute, size_t ws_limit, int out[4]);
 cudaError_t launch_tile(const simt::Params& p, int compute, size_t ws_limit, cudaStream_t s);
 
 }  // namespace tb

@@ -1206,14 +1206,37 @@ bool tile_takes(const simt::Params& p, int compute)
 //   row vectors, binary32 4224 x 8 x 250 49 / 10, but 655k x 38 x 40 245 / 505;
 //     complex 4224 x 8 x 250 61 / 16
 // (contractions of up to 130 stay with the row vectors: 1 to 10 us either way).
+// Up to 8 columns waste most of this kernel's columns or warps, so the narrow
+// ones are ahead as soon as their rows fill the GPU once: binary32 41k x 6 x 68
+// 21 / 80 and 115k x 7 x 269 97 / 139; complex, whose rows are streamed one by
+// one, already 22k x 2 x 245 44 / 63; binary64 where the contraction is short,
+// 286k x 4 x 117 78 / 104, but 109k x 1 x 222 at par and 44k x 3 x 258 58 / 34. From
+// 9 columns the line rises with them: 12 columns 79k x 79 31 / 35, 48k x 337 105 / 87.
 bool tile_over_narrow(const simt::Params& p, int compute, int kind)
 {
     if (!tile_takes(p, compute)) return false;
-    const double rows = (double)p.M * (double)p.L;
-    const bool vectors = kind >= 5;
-    if (compute == TB_R64) return vectors ? p.K >= 64 : p.K > 64;
+    const double rows = (double)p.M * (double)p.L, cols = (double)p.N;
+    const bool vectors = kind >= 5, few = p.N <= 8;
+    if (compute == TB_R64) return few && rows >= 148.0 * 256 ? p.K > 130 : vectors ? p.K >= 64 : p.K > 64;
+    if (compute == TB_C32 && few) return p.K > (vectors ? 130 : 64) && rows < 148.0 * 96;
     if (vectors) return p.K > 130 && rows < 148.0 * 256;
-    return p.K > 64 && (compute == TB_C32 || rows < 148.0 * 1024);
+    if (compute == TB_C32) return p.K > 64 && (p.N > 12 || rows < 148.0 * 1024);
+    if (rows < 148.0 * 256) return p.K > 64;
+    return p.K > 64 && !few && rows < 148.0 * 48 * cols && rows < 148.0 * 1024;
+}
+
+// tile, cluster and splits of a product that this kernel takes
+void tile_describe(const simt::Params& p, int compute, size_t ws_limit, int out[4])
+{
+    tile::with_tile(p, compute, [&](auto w) {
+        using W = decltype(w);
+        const int64_t tiles = ((p.M + W::BM - 1) / W::BM) * ((p.N + W::BN - 1) / W::BN) * p.L;
+        const tile::Split s = tile::choose_split(tiles, p.K, W::BK, p.L * p.M * p.N, W::E, ws_limit);
+        out[0] = W::BM;
+        out[1] = W::BN;
+        out[2] = s.cluster;
+        out[3] = s.splits;
+    });
 }
 
 cudaError_t launch_tile(const simt::Params& p, int compute, size_t ws_limit, cudaStream_t s)

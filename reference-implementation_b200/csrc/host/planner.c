@@ -547,6 +547,9 @@ size_t tb_describe(const tb_plan* p, size_t maxlen, char* out)
                                      "narrow_cvec", "narrow_kt"};
         const int k = tbk_simt_kernel(p);
         if (k >= 0 && k <= 7) at = put(out, maxlen, at, " kernel=%s", kern[k]);
+        int tile[4];
+        if (tbk_simt_tile(p, tile))
+            at = put(out, maxlen, at, " tile=%dx%d cluster=%d splits=%d", tile[0], tile[1], tile[2], tile[3]);
     }
     at = put_modes(out, maxlen, at, "F", &p->F);
     at = put_modes(out, maxlen, at, "K", &p->K);

@@ -87,3 +87,19 @@ def test_rows_fill_more_than_half_a_group(tapp, d, k, types, rows):
 def test_long_unary_modes_take_one_row(tapp, a, types, prec, u, v, rows):
     t = plan_text(tapp, a, "khv", "ah", {"a": 150, "h": 120, "k": 33, "u": u, "v": v}, types, prec)
     assert field(t, "kernel") == "warpdot" and field(t, "rows") == rows, t
+
+
+# up to 8 columns stay with the narrow kernels once their rows fill the GPU, from 9 columns the line rises with them
+@pytest.mark.parametrize("t,prec,m,n,k,kernel", [
+    (TAPP_F32, 0, 57771, 6, 100, "narrow"), (TAPP_F32, 6, 57771, 1, 300, "narrow"), (TAPP_F32, 0, 57771, 9, 100, "tiled"),
+    (TAPP_F32, 0, 57771, 20, 100, "tiled"), (TAPP_F32, 0, 37001, 6, 100, "tiled"), (TAPP_F32, 0, 100001, 9, 100, "narrow"),
+    (TAPP_F32, 0, 100001, 16, 100, "tiled"), (TAPP_F32, 0, 155001, 30, 100, "narrow"), (TAPP_F32, 0, 57771, 20, 64, "narrow"),
+    (TAPP_C32, -1, 22347, 2, 245, "narrow"), (TAPP_C32, -1, 9001, 2, 245, "tiled"), (TAPP_C32, -1, 22347, 9, 245, "tiled"),
+    (TAPP_C32, -1, 278581, 12, 138, "narrow"), (TAPP_C32, -1, 278581, 13, 138, "tiled"),
+    (TAPP_F64, -1, 285869, 4, 117, "narrow"), (TAPP_F64, -1, 285869, 4, 222, "tiled"), (TAPP_F64, -1, 20001, 4, 117, "tiled"),
+    (TAPP_F64, -1, 285869, 9, 117, "tiled")])
+def test_narrow_kernels_keep_few_columns(tapp, t, prec, m, n, k, kernel):
+    text = plan_text(tapp, "mk", "nk", "mn", {"m": m, "n": n, "k": k}, (t,) * 4, prec)
+    got = field(text, "kernel")
+    assert got == kernel or (kernel == "narrow" and got.startswith("narrow")), text
+    assert (field(text, "tile") is not None) == (kernel == "tiled"), text
