@@ -373,7 +373,7 @@ struct Slim32 {
     using T = float;
     static constexpr bool CPLX = false;
     static constexpr int NT = 32 * CT, BM = 256, BN = CT * TN, BK = 8, STAGES = 4, E = 4, PAD = 4;
-    static constexpr int MINB = NT <= 96 ? 4 : NT <= 128 || (NT == 160 && TN == 8) ? 3 : 2;
+    static constexpr int MINB = NT <= 96 ? 4 : NT <= 160 ? 3 : 2;
     static constexpr int LDA = BM + PAD, LDB = BN + PAD;
     uint64_t acc[4][TN / 2][2];
     int row, col;
@@ -440,7 +440,7 @@ struct SlimComplex32 {
     using T = float;
     static constexpr bool CPLX = true;
     static constexpr int NT = 32 * CT, BM = 128, BN = CT * 8, BK = 8, STAGES = 4, E = 8, PAD = 4;
-    static constexpr int MINB = NT <= 96 ? 4 : NT <= 128 ? 3 : 2;
+    static constexpr int MINB = NT <= 96 ? 4 : 2;
     static constexpr int LDA = BM + PAD, LDB = BN + PAD;
     uint64_t acc[4][8];
     int row, col;
@@ -1111,15 +1111,28 @@ static cudaError_t launch(const simt::Params& sp, size_t ws_limit, cudaStream_t 
     return e;
 }
 
-// Tiles by the shorter side N. Up to 64 columns: tall tiles as wide as N
-// rounded up to 8 (binary32 also to 12) where the rows fill the GPU, narrow
-// ones of 128 rows otherwise. Wider: the widest that both sides fill; binary64
-// takes 128 x 64 (two blocks per SM, 32 accumulators a thread), 64 x 64 where
-// M is small.
+// Tiles by the shorter side N. Wide ones where both sides fill them (binary32
+// 128 x 128 and 64 x 64, binary64 128 x 64, two blocks per SM with 32
+// accumulators a thread, or 64 x 64 where M is small), 128 rows of 8 to 64
+// columns for narrow products, and for binary32 and its complex tall tiles as
+// wide as N rounded up to 8 or 12, whose warps own a group of columns each.
+// A block of those has only as many warps as groups, so they need rows for
+// several warps per SM: with fewer, one or two warps an SM wait on every slice
+// (57771 x 2 x 383 165 us, 76 in 128 x 16 tiles). Time in the general tile / in
+// the tall one, 1600 random products: binary32 up to 48 columns 0.3 to 0.8
+// below 4 warps an SM, about 1 at 5, 1.0 to 2.1 from 6 on; 49 to 60 columns 0.6 to
+// 1.0 everywhere (no tall tile), 61 to 64 0.5 to 1.0 below 10 warps, 0.9 to 1.5
+// above. Complex up to 16 columns 0.6 to 1.0 below 2 and 3 warps an SM, 1.1 to 1.4 above,
+// 17 to 24 columns 1.02 to 1.10 from 24 on, 41 to 48 1.05 to 1.18 from 32 on where
+// A lies along the contraction (0.8 to 0.97 else), other widths 0.7 to 1.0.
 template <typename F>
 static auto with_tile(const simt::Params& p, int compute, F&& f)
 {
     const int w8 = (int)((p.N + 7) / 8);
+    // whether full blocks of `rows` rows and `warps` warps put `per_sm` warps on every SM
+    auto fills = [&](int rows, int warps, int per_sm) {
+        return (double)p.M * (double)p.L * warps >= 148.0 * per_sm * rows;
+    };
     switch (compute) {
     case TB_R64:
         if (p.N > 64) {
@@ -1137,36 +1150,23 @@ static auto with_tile(const simt::Params& p, int compute, F&& f)
         default: return f(Real64<128, 64, 4, 2, 2>());
         }
     case TB_C32:
-        if (p.N <= 64 && (double)p.M * (double)p.L >= 148.0 * 128) {
-            switch (w8) {
-            case 1: return f(SlimComplex32<1>());
-            case 2: return f(SlimComplex32<2>());
-            case 3: return f(SlimComplex32<3>());
-            case 4: return f(SlimComplex32<4>());
-            case 5: return f(SlimComplex32<5>());
-            case 6: return f(SlimComplex32<6>());
-            case 7: return f(SlimComplex32<7>());
-            default: return f(SlimComplex32<8>());
-            }
-        }
+        if (p.N <= 8 && fills(128, 1, 2)) return f(SlimComplex32<1>());
+        if (p.N > 8 && p.N <= 16 && fills(128, 2, 3)) return f(SlimComplex32<2>());
+        if (p.N > 16 && p.N <= 24 && fills(128, 3, 24)) return f(SlimComplex32<3>());
+        if (p.N > 40 && p.N <= 48 && !p.a_rows_fast && fills(128, 6, 32)) return f(SlimComplex32<6>());
         if (p.N <= 32) return f(Complex32<128, 32>());
         return f(Complex32<64, 64>());
     case TB_C64:
         if (p.N <= 32) return f(Complex64<128, 32, 4, 2>());
         return f(Complex64<64, 64, 2, 4>());
     default:
-        if (p.N <= 64 && (double)p.M * (double)p.L >= 148.0 * 256) {
-            if (p.N <= 8) return f(Slim32<1, 8>());
-            if (p.N <= 12) return f(Slim32<1, 12>());
-            if (p.N <= 16) return f(Slim32<2, 8>());
-            if (p.N <= 24) return f(Slim32<2, 12>());
-            if (p.N <= 32) return f(Slim32<4, 8>());
-            if (p.N <= 36) return f(Slim32<3, 12>());
-            if (p.N <= 40) return f(Slim32<5, 8>());
-            if (p.N <= 48) return f(Slim32<4, 12>());
-            if (p.N <= 60) return f(Slim32<5, 12>());
-            return f(Slim32<8, 8>());
-        }
+        if (p.N <= 12 && fills(256, 1, 6)) return p.N <= 8 ? f(Slim32<1, 8>()) : f(Slim32<1, 12>());
+        if (p.N > 12 && p.N <= 24 && fills(256, 2, 6)) return p.N <= 16 ? f(Slim32<2, 8>()) : f(Slim32<2, 12>());
+        if (p.N > 24 && p.N <= 32 && fills(256, 4, 6)) return f(Slim32<4, 8>());
+        if (p.N > 32 && p.N <= 36 && fills(256, 3, 5)) return f(Slim32<3, 12>());
+        if (p.N > 36 && p.N <= 40 && fills(256, 5, 6)) return f(Slim32<5, 8>());
+        if (p.N > 40 && p.N <= 48 && fills(256, 4, 6)) return f(Slim32<4, 12>());
+        if (p.N > 60 && p.N <= 64 && fills(256, 8, 10)) return f(Slim32<8, 8>());
         if (p.N <= 16) return f(Real32<128, 16, 4, 2, 2>());
         if (p.N <= 32) return f(Real32<128, 32, 4, 4, 2>());
         if (p.M > 64 && p.N > 64 && (double)p.M * (double)p.N * (double)p.L >= 148.0 * 128 * 128)
@@ -1211,7 +1211,8 @@ bool tile_takes(const simt::Params& p, int compute)
 // 21 / 80 and 115k x 7 x 269 97 / 139; complex, whose rows are streamed one by
 // one, already 22k x 2 x 245 44 / 63; binary64 where the contraction is short,
 // 286k x 4 x 117 78 / 104, but 109k x 1 x 222 at par and 44k x 3 x 258 58 / 34. From
-// 9 columns the line rises with them: 12 columns 79k x 79 31 / 35, 48k x 337 105 / 87.
+// 9 columns the line rises with them: 12 columns 79k x 79 31 / 35, 48k x 337 105 / 87,
+// 16 columns 113k x 231 89 / 107.
 bool tile_over_narrow(const simt::Params& p, int compute, int kind)
 {
     if (!tile_takes(p, compute)) return false;
@@ -1222,7 +1223,8 @@ bool tile_over_narrow(const simt::Params& p, int compute, int kind)
     if (vectors) return p.K > 130 && rows < 148.0 * 256;
     if (compute == TB_C32) return p.K > 64 && (p.N > 12 || rows < 148.0 * 1024);
     if (rows < 148.0 * 256) return p.K > 64;
-    return p.K > 64 && !few && rows < 148.0 * 48 * cols && rows < 148.0 * 1024;
+    // (from 13 columns tall tiles take over where the rows fill them)
+    return p.K > 64 && !few && rows < 148.0 * 1024 && (rows < 148.0 * 40 * cols || (p.N > 12 && rows >= 148.0 * 768));
 }
 
 // tile, cluster and splits of a product that this kernel takes

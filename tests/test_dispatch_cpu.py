@@ -91,9 +91,9 @@ def test_long_unary_modes_take_one_row(tapp, a, types, prec, u, v, rows):
 
 # up to 8 columns stay with the narrow kernels once their rows fill the GPU, from 9 columns the line rises with them
 @pytest.mark.parametrize("t,prec,m,n,k,kernel", [
-    (TAPP_F32, 0, 57771, 6, 100, "narrow"), (TAPP_F32, 6, 57771, 1, 300, "narrow"), (TAPP_F32, 0, 57771, 9, 100, "tiled"),
+    (TAPP_F32, 0, 57771, 6, 100, "narrow"), (TAPP_F32, 6, 57771, 1, 300, "narrow"), (TAPP_F32, 0, 50001, 9, 100, "tiled"),
     (TAPP_F32, 0, 57771, 20, 100, "tiled"), (TAPP_F32, 0, 37001, 6, 100, "tiled"), (TAPP_F32, 0, 100001, 9, 100, "narrow"),
-    (TAPP_F32, 0, 100001, 16, 100, "tiled"), (TAPP_F32, 0, 155001, 30, 100, "narrow"), (TAPP_F32, 0, 57771, 20, 64, "narrow"),
+    (TAPP_F32, 0, 100001, 16, 100, "narrow"), (TAPP_F32, 0, 90001, 16, 100, "tiled"), (TAPP_F32, 0, 120001, 16, 100, "tiled"), (TAPP_F32, 0, 155001, 30, 100, "narrow"), (TAPP_F32, 0, 57771, 20, 64, "narrow"),
     (TAPP_C32, -1, 22347, 2, 245, "narrow"), (TAPP_C32, -1, 9001, 2, 245, "tiled"), (TAPP_C32, -1, 22347, 9, 245, "tiled"),
     (TAPP_C32, -1, 278581, 12, 138, "narrow"), (TAPP_C32, -1, 278581, 13, 138, "tiled"),
     (TAPP_F64, -1, 285869, 4, 117, "narrow"), (TAPP_F64, -1, 285869, 4, 222, "tiled"), (TAPP_F64, -1, 20001, 4, 117, "tiled"),
@@ -103,3 +103,18 @@ def test_narrow_kernels_keep_few_columns(tapp, t, prec, m, n, k, kernel):
     got = field(text, "kernel")
     assert got == kernel or (kernel == "narrow" and got.startswith("narrow")), text
     assert (field(text, "tile") is not None) == (kernel == "tiled"), text
+
+
+# tall tiles need rows for several warps an SM, and there are none where general ones do better
+@pytest.mark.parametrize("t,m,n,tile", [
+    (TAPP_F32, 57771, 12, "128x16"), (TAPP_F32, 230000, 12, "256x12"), (TAPP_F32, 100001, 20, "128x32"),
+    (TAPP_F32, 120001, 20, "256x24"), (TAPP_F32, 50001, 33, "64x64"), (TAPP_F32, 70001, 33, "256x36"),
+    (TAPP_F32, 50001, 40, "256x40"), (TAPP_F32, 60001, 48, "256x48"), (TAPP_F32, 500001, 50, "64x64"),
+    (TAPP_F32, 500001, 60, "64x64"), (TAPP_F32, 40001, 64, "64x64"), (TAPP_F32, 60001, 64, "256x64"),
+    (TAPP_C32, 30001, 8, "128x32"), (TAPP_C32, 40001, 8, "128x8"), (TAPP_C32, 20001, 16, "128x32"), (TAPP_C32, 30001, 16, "128x16"),
+    (TAPP_C32, 100001, 24, "128x32"), (TAPP_C32, 160001, 24, "128x24"), (TAPP_C32, 500001, 25, "128x32"),
+    (TAPP_C32, 500001, 40, "64x64"), (TAPP_C32, 500001, 45, "64x64")])
+def test_tall_tiles_need_rows(tapp, t, m, n, tile):
+    # a contraction beyond what the narrow kernels hold
+    text = plan_text(tapp, "mk", "nk", "mn", {"m": m, "n": n, "k": 5000}, (t,) * 4, -1)
+    assert (field(text, "kernel"), field(text, "tile")) == ("tiled", tile), text
