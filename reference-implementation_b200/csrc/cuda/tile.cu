@@ -33,7 +33,7 @@
 // of a thread-block cluster (2, 4 or 8), whose partial tiles meet through
 // distributed shared memory and are added in rank order, each block finishing
 // its share of the tile: no workspace and no second launch. Where 8 ranks
-// would each still walk more than 16 slices, the splits go to a workspace
+// would each still walk more than some 10 slices, the splits go to a workspace
 // and k_tile_final adds them in order. Both orders are fixed: a product gives
 // the same bits in every run, alone or served.
 #include <cstdio>
@@ -986,10 +986,15 @@ struct Split {
 
 // About two blocks per SM in all. A split keeps at least two slices of the
 // contraction (less would spend more on the meeting of the ranks than on the
-// sums); a cluster serves up to 8, beyond that the workspace pays once every
-// one of 8 ranks would walk more than 16 slices. ws_limit: the scratch a
-// product is charged for by a server (simt_scratch_bytes), which the
-// workspace stays within.
+// sums); a cluster serves up to 8, beyond that the workspace and its second
+// launch pay once every one of 8 ranks would walk more than 11 slices (binary32),
+// 10 (binary64, complex) or 8 (complex binary64). 8 ranks / workspace, us: binary32
+// 1384 terms 16.6 / 17.8, 1660 terms 16.3 / 13.4; complex 1029 terms 38.5 / 42.9, 1338
+// terms 29.2 / 18.4; binary64 1262 terms 12.1 / 12.9, 1329 terms 17.4 / 13.7; complex
+// binary64 570 terms 23 / 21, 1811 terms 57.6 / 29.7; 16 slices where fewer than 16
+// splits fill the GPU (32 tiles, 1651 terms 26.3 / 33.4). ws_limit: the scratch a
+// product is charged for by a server (simt_scratch_bytes), which the workspace
+// stays within.
 static Split choose_split(int64_t tiles, int64_t K, int bk, int64_t outs, size_t elem, size_t ws_limit)
 {
     Split r = {1, 1, K, 0};
@@ -997,7 +1002,8 @@ static Split choose_split(int64_t tiles, int64_t K, int bk, int64_t outs, size_t
     r.chunk = slices * bk;
     if (tiles >= 148 || slices < 4) return r;
     const int64_t want = (2 * 148 + tiles - 1) / tiles;
-    if (want > 8 && slices > 8 * 16) {
+    const int most = want < 16 ? 16 : elem == 4 ? 11 : elem == 8 ? 10 : 8;
+    if (want > 8 && slices > 8 * most) {
         int64_t S = want < slices / 4 ? want : slices / 4;
         if (S > 1024) S = 1024;
         while (S > 1 && (double)S * (double)outs * (double)elem > (double)ws_limit) S /= 2;

@@ -118,3 +118,14 @@ def test_tall_tiles_need_rows(tapp, t, m, n, tile):
     # a contraction beyond what the narrow kernels hold
     text = plan_text(tapp, "mk", "nk", "mn", {"m": m, "n": n, "k": 5000}, (t,) * 4, -1)
     assert (field(text, "kernel"), field(text, "tile")) == ("tiled", tile), text
+
+
+# few tiles and a long contraction: splits through the workspace once 8 ranks of a cluster would walk some 10 slices each
+@pytest.mark.parametrize("t,m,n,k,through_workspace", [
+    (TAPP_C64, 384, 14, 1811, True), (TAPP_C64, 384, 14, 1025, True), (TAPP_C64, 384, 14, 1024, False),
+    (TAPP_C32, 136, 38, 1903, True), (TAPP_C32, 136, 38, 1280, False), (TAPP_F64, 56, 91, 1400, True),
+    (TAPP_F64, 56, 91, 1280, False), (TAPP_F32, 108, 37, 1420, True), (TAPP_F32, 108, 37, 1400, False), (TAPP_F32, 2048, 33, 1660, False)])
+def test_long_contractions_of_few_tiles_are_split(tapp, t, m, n, k, through_workspace):
+    text = plan_text(tapp, "mk", "nk", "mn", {"m": m, "n": n, "k": k}, (t,) * 4, -1, path=tapp_b200.PATH_SIMT)
+    assert field(text, "kernel") == "tiled", text
+    assert (int(field(text, "splits")) > 8, int(field(text, "cluster"))) == (through_workspace, 1 if through_workspace else 8), text
