@@ -984,7 +984,10 @@ struct Split {
     size_t ws_bytes;
 };
 
-// About two blocks per SM in all. A split keeps at least two slices of the
+// About two blocks per SM in all; products of 148 tiles and more are not split,
+// but for those of up to one and a half tiles per SM and more than 32 slices, in
+// which half the SMs would wait for a second whole tile (160 tiles, 2909 terms 259
+// / 213 us in two ranks; with 64 to 130 terms 0.74 to 0.96 of the speed). A split keeps at least two slices of the
 // contraction (less would spend more on the meeting of the ranks than on the
 // sums); a cluster serves up to 8, beyond that the workspace and its second
 // launch pay once every one of 8 ranks would walk more than 11 slices (binary32),
@@ -1000,7 +1003,7 @@ static Split choose_split(int64_t tiles, int64_t K, int bk, int64_t outs, size_t
     Split r = {1, 1, K, 0};
     const int64_t slices = (K + bk - 1) / bk;
     r.chunk = slices * bk;
-    if (tiles >= 148 || slices < 4) return r;
+    if (tiles >= 222 || (tiles >= 148 && slices <= 32) || slices < 4) return r;
     const int64_t want = (2 * 148 + tiles - 1) / tiles;
     const int most = want < 16 ? 16 : elem == 4 ? 11 : elem == 8 ? 10 : 8;
     if (want > 8 && slices > 8 * most) {

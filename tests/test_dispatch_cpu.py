@@ -129,3 +129,11 @@ def test_long_contractions_of_few_tiles_are_split(tapp, t, m, n, k, through_work
     text = plan_text(tapp, "mk", "nk", "mn", {"m": m, "n": n, "k": k}, (t,) * 4, -1, path=tapp_b200.PATH_SIMT)
     assert field(text, "kernel") == "tiled", text
     assert (int(field(text, "splits")) > 8, int(field(text, "cluster"))) == (through_workspace, 1 if through_workspace else 8), text
+
+
+# from one to one and a half tiles per SM, long contractions are shared by two ranks
+@pytest.mark.parametrize("t,l,k,cluster", [(TAPP_F32, 40, 900, 2), (TAPP_F32, 40, 512, 1), (TAPP_F32, 55, 900, 2), (TAPP_F32, 56, 900, 1),
+                                           (TAPP_F64, 80, 900, 2), (TAPP_C64, 40, 900, 2)])
+def test_little_more_than_a_tile_per_sm(tapp, t, l, k, cluster):
+    text = plan_text(tapp, "mkl", "nkl", "mnl", {"m": 106, "n": 86, "k": k, "l": l}, (t,) * 4, -1)
+    assert field(text, "kernel") == "tiled" and int(field(text, "cluster")) == cluster, text
