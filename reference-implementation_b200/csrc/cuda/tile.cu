@@ -1120,11 +1120,17 @@ static cudaError_t launch(const simt::Params& sp, size_t ws_limit, cudaStream_t 
     return e;
 }
 
-// Tiles by the shorter side N. Wide ones where both sides fill them (binary32
-// 128 x 128 and 64 x 64, binary64 128 x 64, two blocks per SM with 32
-// accumulators a thread, or 64 x 64 where M is small), 128 rows of 8 to 64
-// columns for narrow products, and for binary32 and its complex tall tiles as
-// wide as N rounded up to 8 or 12, whose warps own a group of columns each.
+// Tiles by the shorter side N. Wide ones where both sides fill them (binary64
+// 128 x 64, two blocks per SM with 32 accumulators a thread, or 64 x 64 where M
+// is small; binary32 128 x 128 with two tiles per SM and, shared by the ranks of
+// a cluster, with fewer where the contraction is long, sooner if operands lie
+// along it: a 64 x 64 tile reads twice the shared memory per multiply-add and
+// copies transposing, element by element, twice as often. 64 x 64 / 128 x 128,
+// us: 634 x 480 x 2832 126 / 77, 817 x 1168 x 1972 in 2 batches, both operands along
+// the contraction, 411 / 290; mean of 350 products 1.1 to 1.4 times from the lines
+// on, 0.5 to 1.1 below them and with fewer than 16 tiles), 128 rows of 8 to 64 columns for narrow products, and for binary32 and its
+// complex tall tiles as wide as N rounded up to 8 or 12, whose warps own a group
+// of columns each.
 // A block of those has only as many warps as groups, so they need rows for
 // several warps per SM: with fewer, one or two warps an SM wait on every slice
 // (57771 x 2 x 383 165 us, 76 in 128 x 16 tiles). Time in the general tile / in
@@ -1178,8 +1184,13 @@ static auto with_tile(const simt::Params& p, int compute, F&& f)
         if (p.N > 60 && p.N <= 64 && fills(256, 8, 10)) return f(Slim32<8, 8>());
         if (p.N <= 16) return f(Real32<128, 16, 4, 2, 2>());
         if (p.N <= 32) return f(Real32<128, 32, 4, 4, 2>());
-        if (p.M > 64 && p.N > 64 && (double)p.M * (double)p.N * (double)p.L >= 148.0 * 128 * 128)
-            return f(Real32<128, 128, 8, 8, 2>());
+        if (p.M > 64 && p.N > 64) {
+            const double tiles = (double)((p.M + 127) / 128) * (double)((p.N + 127) / 128) * (double)p.L;
+            const int along_k = !p.a_rows_fast + !p.b_rows_fast;
+            if ((double)p.M * (double)p.N * (double)p.L >= 148.0 * 128 * 128 ||
+                (tiles >= 16 && (along_k == 2 ? p.K >= 512 : p.K >= 1024 && (along_k || p.K >= 2048 || tiles < 128))))
+                return f(Real32<128, 128, 8, 8, 2>());
+        }
         return f(Real32<64, 64, 4, 4, 2>());
     }
 }
@@ -1187,7 +1198,12 @@ static auto with_tile(const simt::Params& p, int compute, F&& f)
 }  // namespace tile
 
 // Operands stored as the type they are computed in; binary32 may also be
-// rounded to 16 bits. Coordinates fit 32-bit division.
+// rounded to 16 bits. Coordinates fit 32-bit division. Two binary32 operands in
+// 16-byte runs along a contraction of 1536 terms and more stay with k_simt, which
+// loads four terms at once where this kernel copies one, as long as they have
+// fewer than two 128 x 128 tiles per SM but more than 5 (k_simt / this kernel,
+// us: 837 x 101 x 2416 38 / 48, 94 x 1773 x 1680 42 / 55, 392 x 68 x 42668 in 2
+// batches 322 / 622, 1.04 on average; with 4 tiles 154 x 144 x 3720 52 / 24).
 bool tile_takes(const simt::Params& p, int compute)
 {
     static const int stored[4] = {T_F32, T_F64, T_C32, T_C64};  // by TB_R32 .. TB_C64
@@ -1199,6 +1215,10 @@ bool tile_takes(const simt::Params& p, int compute)
     const simt::Modes* m[9] = {&p.am, &p.ak, &p.al, &p.bn, &p.bk, &p.bl, &p.cm, &p.cn, &p.cl};
     for (int j = 0; j < 9; j++)
         if (m[j]->n > tile::MAXM) return false;
+    if (compute == TB_R32 && p.a_vec && p.b_vec && !p.a_rows_fast && !p.b_rows_fast && p.M > 64 && p.N > 64 && p.K >= 1536) {
+        const double tiles = (double)((p.M + 127) / 128) * (double)((p.N + 127) / 128) * (double)p.L;
+        if (tiles >= 6 && (double)p.M * (double)p.N * (double)p.L < 148.0 * 128 * 128) return false;
+    }
     return true;
 }
 

@@ -137,3 +137,17 @@ def test_long_contractions_of_few_tiles_are_split(tapp, t, m, n, k, through_work
 def test_little_more_than_a_tile_per_sm(tapp, t, l, k, cluster):
     text = plan_text(tapp, "mkl", "nkl", "mnl", {"m": 106, "n": 86, "k": k, "l": l}, (t,) * 4, -1)
     assert field(text, "kernel") == "tiled" and int(field(text, "cluster")) == cluster, text
+
+
+# binary32 tiles of 128 x 128 also for fewer tiles where the contraction is long or an operand lies along it; both operands
+# in 16-byte runs along a long contraction go to the kernel that loads runs (no tile)
+@pytest.mark.parametrize("a,b,m,n,k,tile", [
+    ("mk", "nk", 634, 480, 2832, "128x128"), ("mk", "nk", 634, 480, 1100, "128x128"), ("mk", "nk", 634, 480, 900, "64x64"),
+    ("mk", "nk", 200, 180, 2832, "64x64"), ("mk", "nk", 634, 60, 2832, "64x64"), ("mk", "nk", 2000, 2000, 100, "128x128"),
+    ("mk", "nk", 1500, 1400, 1100, "64x64"), ("km", "nk", 1500, 1400, 1100, "128x128"), ("mk", "kn", 1500, 1400, 1000, "64x64"),
+    ("km", "kn", 634, 480, 512, "128x128"), ("km", "kn", 634, 480, 508, "64x64"), ("km", "kn", 300, 200, 600, "64x64"),
+    ("km", "kn", 634, 480, 1536, None), ("km", "kn", 634, 480, 1537, "128x128"), ("km", "kn", 634, 480, 1532, "128x128"),
+    ("km", "kn", 300, 200, 2048, None), ("km", "kn", 200, 200, 2048, "64x64"), ("km", "kn", 2000, 2000, 2048, "128x128")])
+def test_wide_tiles_for_fewer_tiles(tapp, a, b, m, n, k, tile):
+    text = plan_text(tapp, a, b, "mn", {"m": m, "n": n, "k": k}, (TAPP_F32,) * 4, 0, path=tapp_b200.PATH_SIMT)
+    assert field(text, "tile") == tile, text
