@@ -814,6 +814,7 @@ __global__ void __launch_bounds__(W::NT, W::MINB) k_tile(const __grid_constant__
     const int ranks = p.cluster;
     if (ranks > 1) cluster_barrier();
     else __syncthreads();
+    static_assert(BM * BN % 8 == 0, "equal shares of a tile for 2, 4 and 8 ranks");
     const int share = BM * BN / ranks, first = ranks > 1 ? (int)blockIdx.y * share : 0;
     // the sum of the ranks' partial results for output (r, c), in rank order
     auto summed = [&](int r, int c) {
@@ -857,7 +858,8 @@ __global__ void __launch_bounds__(W::NT, W::MINB) k_tile(const __grid_constant__
             const longlong2* outer = RF ? colCD : rowCD;
             const int n_in = RF ? rows_a : rows_b, n_out = RF ? rows_b : rows_a;
             const int o0 = ranks > 1 ? (int)blockIdx.y * (OUT / ranks) : 0;
-            const int o1 = min(n_out, ranks > 1 ? o0 + OUT / ranks : OUT);
+            // the last rank finishes what the ranks' equal shares leave (a width of 12 has no eighths)
+            const int o1 = min(n_out, ranks > 1 && (int)blockIdx.y + 1 < ranks ? o0 + OUT / ranks : OUT);
             const int lane = t & 31;
             int64_t ic[IT], id[IT];
 #pragma unroll
