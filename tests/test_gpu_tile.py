@@ -88,8 +88,8 @@ def test_same_bits_every_run(tapp, gpu, storage, M, N, K):
     assert tapp_b200.load().launches() > 0
 
 
-# the tall tiles: every width of 8 or 12 columns a group, with remainders in columns, rows and contraction, rows in
-# 16-byte groups, in pairs, alone and across the contraction
+# products of many rows and up to 64 columns, with remainders in columns, rows and contraction, in whichever narrow or
+# tiled kernel the rules give them (test_gpu_tile_forms.py has every tall tile)
 @pytest.mark.parametrize("storage,prec", [(0, 0), (0, 6), (1, -1), (2, -1)])
 @pytest.mark.parametrize("N", [1, 8, 11, 16, 23, 31, 36, 39, 48, 59, 64])
 @pytest.mark.parametrize("M,a_t", [(38004, 0), (38002, 0), (37999, 0), (37999, 1)])
