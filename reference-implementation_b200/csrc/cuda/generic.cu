@@ -254,7 +254,7 @@ __device__ __forceinline__ void element(const GenParams& p, const void* A, const
 // one output at a time, of the grouped launches and of the request loop.
 // One output per thread was bound by one load of the varying operand in flight
 // for each of the shared one, one per warp by index arithmetic and shuffles:
-// the 823 MB Hadamard product of 69 terms went from 621 to 199 us (4.1 TB/s),
+// the 823 MB Hadamard product of 69 terms went from 621 to 209 us (3.9 TB/s),
 // its form with the contraction contiguous from 1790 to 331 us, and the
 // mixed-class product's unary sums, loads side by side and offsets from tables,
 // from 40 to 17 us.

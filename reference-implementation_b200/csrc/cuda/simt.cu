@@ -1,9 +1,10 @@
 // CUDA-core products in the turned L/M/N/K view. k_simt is the tiled GEMM for
 // operands that are converted as they are loaded (storage other than the
 // compute type, complex operands rounded to 16 bits, more than 8 modes in an
-// index class or coordinates beyond 31 bits); operands stored as they are
-// computed with go to k_tile (tile.cu), and narrow products to the kernels
-// further down.
+// index class or coordinates beyond 31 bits) and for binary32 operands in
+// 16-byte runs along a long contraction (tile_takes); other operands stored as
+// they are computed with go to k_tile (tile.cu), and narrow products to the
+// kernels further down.
 // Complex operands keep real and imaginary planes in shared memory and
 // accumulate with four FMAs per product; op_A/op_B conjugation is applied at
 // load, op_C and op_D in the epilogue.

@@ -456,13 +456,11 @@ static int num_sms();
 // blocks start while that pack's last blocks drain. The packs read only the
 // product's operands, which the stream work before the first pack produced.
 template <typename K, typename... Args>
-static void launch_pack_kernel(K kern, dim3 grid, unsigned threads, size_t smem, cudaStream_t s, bool pdl,
-                               Args... args)
+static void launch_pack_kernel(K kern, dim3 grid, unsigned threads, cudaStream_t s, bool pdl, Args... args)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(threads, 1, 1);
-    cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -488,7 +486,7 @@ static void launch_pack_vec(const PackParams& pp, int64_t lz, cudaStream_t s, bo
     dv.lsz = make_fastdiv((uint32_t)std::max<int64_t>(pp.Lsz, 1));
     const int64_t grid = tiles_r * tiles_k * lz;
     if (grid > 0)
-        launch_pack_kernel(rf ? k_pack_cols<SPLIT, FMT> : k_pack_runs<SPLIT, FMT>, dim3((unsigned)grid), PR_THREADS, 0, s, pdl,
+        launch_pack_kernel(rf ? k_pack_cols<SPLIT, FMT> : k_pack_runs<SPLIT, FMT>, dim3((unsigned)grid), PR_THREADS, s, pdl,
                            pp, dv);
 }
 
@@ -516,10 +514,10 @@ static void launch_pack_vec3(const PackParams& pp, int split, int fmt, int64_t l
 template <typename T, bool RF>
 static void launch_pack_real3(const PackParams& pp, int split, int fmt, dim3 grid, cudaStream_t s, bool pdl)
 {
-    if (split == 3) launch_pack_kernel(k_pack_real<T, 3, 0, RF>, grid, 256, 0, s, pdl, pp);
-    else if (split == 2) launch_pack_kernel(k_pack_real<T, 2, 0, RF>, grid, 256, 0, s, pdl, pp);
-    else if (fmt == 1) launch_pack_kernel(k_pack_real<T, 1, 1, RF>, grid, 256, 0, s, pdl, pp);
-    else launch_pack_kernel(k_pack_real<T, 1, 0, RF>, grid, 256, 0, s, pdl, pp);
+    if (split == 3) launch_pack_kernel(k_pack_real<T, 3, 0, RF>, grid, 256, s, pdl, pp);
+    else if (split == 2) launch_pack_kernel(k_pack_real<T, 2, 0, RF>, grid, 256, s, pdl, pp);
+    else if (fmt == 1) launch_pack_kernel(k_pack_real<T, 1, 1, RF>, grid, 256, s, pdl, pp);
+    else launch_pack_kernel(k_pack_real<T, 1, 0, RF>, grid, 256, s, pdl, pp);
 }
 
 // whether a mode list's first mode has stride 1 and extent % 4 == 0 and all

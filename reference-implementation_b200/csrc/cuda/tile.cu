@@ -4,9 +4,9 @@
 //
 //   D[l,m,n] = op_D(alpha * sum_k A[l,m,k] B[l,k,n] + beta * op_C(C[l,m,n]))
 //
-// Operands are gathered in place, from any strides. A block of 256 threads
-// owns a BM x BN tile; per BK-deep slice of the contraction every thread
-// copies its share of the two operand tiles with cp.async into a ring of
+// Operands are gathered in place, from any strides. A block (256 threads, 32
+// to 256 for the tall tiles) owns a BM x BN tile; per BK-deep slice of the
+// contraction every thread copies its share of the two operand tiles with cp.async into a ring of
 // STAGES slices, [k][row] in shared memory whatever the operand's own order:
 //   - rows contiguous, in 16-byte groups: one 16-byte copy per group;
 //   - rows nearest, any alignment: one copy per element, lanes along rows;
@@ -14,8 +14,8 @@
 //     32-byte runs of several rows, so that whole sectors are read and the
 //     transposed writes fall on different banks (row length BM + PAD).
 // The offsets of the contracted coordinates come from a table in shared
-// memory that all threads refill 8 slices at a time, four slices before its
-// first use, so no index arithmetic stands between two slices. (The kernel
+// memory that all threads refill BATCH slices at a time, BATCH / 2 slices before
+// its first use, so no index arithmetic stands between two slices. (The kernel
 // before, which loaded through registers and resolved each slice's offsets
 // between two barriers, ran 4096^3 binary32 in 3.75 ms: 0.49 of the FMA pipe.)
 //
