@@ -2346,13 +2346,25 @@ static int narrow_kind(const tb_plan* P, const simt::Params& p, int nb)
     return narrow_choice(p, nb, P->compute == TB_R32 ? 4 : 8).kind;
 }
 
+// Whether k_tile takes a product that a narrow kernel could run, by its layout
+// alone, as if every buffer were aligned: the ranks of a cluster add in another
+// order than a narrow kernel's thread, and where a caller's buffers lie must
+// not show in the product's bits.
+static bool tile_over_narrow_layout(const tb_plan* P, const simt::Params& p, int nb)
+{
+    simt::Params q = p;
+    q.A = q.B = q.C = nullptr;
+    q.D = nullptr;
+    return tile_over_narrow(q, P->compute, narrow_kind(P, q, nb));
+}
+
 cudaError_t launch_simt(const tb_plan* P, const tb_ptrs* d, cudaStream_t s)
 {
     using namespace simt;
     Params p;
     simt_params(P, d, p);
     const int nb = narrow_width(P, p);
-    if (nb && !tile_over_narrow(p, P->compute, narrow_kind(P, p, nb))) {
+    if (nb && !tile_over_narrow_layout(P, p, nb)) {
         NarrowParams np;
         memset(&np, 0, sizeof(np));
         np.p = p;

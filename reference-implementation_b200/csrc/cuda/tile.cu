@@ -963,8 +963,8 @@ static void map2(Map2& m, const simt::Modes& s)
     }
 }
 
-// Whether groups of w neighbouring rows are `bytes` aligned bytes: the first
-// row mode has stride 1 and an extent divisible by w, and every other stride
+// Whether groups of w neighbouring rows (or contracted values) are `bytes`
+// aligned bytes: their first mode has stride 1 and an extent divisible by w, and every other stride
 // and the base keep the alignment.
 static bool rows_in_groups(const simt::Modes& rows, const simt::Modes& ks, const simt::Modes& ls, const void* base, int w,
                            int bytes)
@@ -1217,7 +1217,9 @@ bool tile_takes(const simt::Params& p, int compute)
     const simt::Modes* m[9] = {&p.am, &p.ak, &p.al, &p.bn, &p.bk, &p.bl, &p.cm, &p.cn, &p.cl};
     for (int j = 0; j < 9; j++)
         if (m[j]->n > tile::MAXM) return false;
-    if (compute == TB_R32 && p.a_vec && p.b_vec && !p.a_rows_fast && !p.b_rows_fast && p.M > 64 && p.N > 64 && p.K >= 1536) {
+    // (by the layout alone: where the buffers lie must not choose another order of the sums)
+    if (compute == TB_R32 && !p.a_rows_fast && !p.b_rows_fast && p.M > 64 && p.N > 64 && p.K >= 1536 &&
+        tile::rows_in_groups(p.ak, p.am, p.al, nullptr, 4, 16) && tile::rows_in_groups(p.bk, p.bn, p.bl, nullptr, 4, 16)) {
         const double tiles = (double)((p.M + 127) / 128) * (double)((p.N + 127) / 128) * (double)p.L;
         if (tiles >= 6 && (double)p.M * (double)p.N * (double)p.L < 148.0 * 128 * 128) return false;
     }

@@ -88,3 +88,28 @@ def test_other_storage_of_c_and_d(tapp, oracle, gpu, types, prec, M, N, K, clust
     if splits is None:
         assert int(field(text, "splits")) > 1, text
     check(tapp, oracle, case, **{k: v for k, v in (("cluster", cluster), ("splits", splits)) if v})
+
+
+# where the buffers lie does not show in the bits: the same product 16-byte aligned and aligned to its elements only
+@pytest.mark.parametrize("labels,ext,storage", [(("mk", "nk", "mn"), {"m": 10000, "n": 30, "k": 100}, 0),
+                                                (("mk", "nk", "mn"), {"m": 3000, "n": 20, "k": 64}, 1),
+                                                (("km", "kn", "mn"), {"m": 634, "n": 480, "k": 1536}, 0)])
+def test_bits_do_not_depend_on_alignment(tapp, gpu, labels, ext, storage):
+    import torch
+    e, i = (lambda x: [ext[c] for c in x]), (lambda x: [ord(c) for c in x])
+    case = spec_case(np.random.default_rng(9), storage, -1, tuple(e(x) for x in labels + labels[2:]),
+                     tuple(i(x) for x in labels + labels[2:]))
+    got = []
+    for shift in (0, case.A.itemsize):
+        dev, ptrs = [], []
+        for t in (case.A, case.B, case.C, case.D):
+            raw = np.zeros(t.buf.nbytes + shift, dtype=np.uint8)
+            raw[shift:] = t.buf.view(np.uint8)
+            dev.append(torch.from_numpy(raw).cuda())
+            ptrs.append(dev[-1].data_ptr() + shift + t.base * t.itemsize)
+        ex = simt_executor(tapp)
+        assert case.run(tapp, executor=ex, A_ptr=ptrs[0], B_ptr=ptrs[1], C_ptr=ptrs[2], D_ptr=ptrs[3]) == 0
+        torch.cuda.synchronize()
+        tapp.lib.TAPP_destroy_executor(ex)
+        got.append(dev[3].cpu().numpy()[shift:].tobytes())
+    assert got[0] == got[1]
